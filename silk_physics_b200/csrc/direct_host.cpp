@@ -1,0 +1,265 @@
+// Host side of the direct ADMM solve (see direct_system.hpp).
+#include <algorithm>
+
+#include "direct_system.hpp"
+
+namespace silkb {
+
+namespace {
+
+constexpr int kWarps = kDirectThreads / 32;
+constexpr size_t kSolveSmem = 128 * 1024;  // gathered vectors of a block
+
+// Warps that share a task: as many as fill the chip in one round of tasks
+// while each still has eight rows, and enough that the gathered vectors of
+// a block's groups fit its shared memory.
+int group_warps(int tasks, int rows, int sms) {
+  int g = 32;
+  for (int c : {1, 4, 8, 16})
+    if ((int64_t)tasks * c * 2 > (int64_t)sms * kWarps || rows <= 8 * c) {
+      g = c;
+      break;
+    }
+  while (g < 32 && (size_t)(kWarps / g) * rows * sizeof(float4) > kSolveSmem)
+    g = g == 1 ? 4 : 2 * g;
+  return g;
+}
+
+}  // namespace
+
+DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
+                           cudaStream_t st) {
+  std::vector<float> pos(3 * (size_t)S.nv);
+  for (int i = 0; i < S.nv; ++i)
+    for (int d = 0; d < 3; ++d) pos[3 * (size_t)S.perm[i] + d] = rest[3 * (size_t)i + d];
+  DirectPlan P;
+  if (!build_direct_plan(S.nv, S.Lrows, S.Lcols, pos, P)) return;
+  const int nl = P.levels();
+  if (nl > kDirectMaxLevels) return;
+  int64_t front[2] = {0, 0};
+  int panel = 0, level_nodes = 0;
+  for (int l = 0; l < nl; ++l) {
+    front[l & 1] = std::max(front[l & 1], P.level_front[l]);
+    panel = std::max(panel, P.level_panel[l]);
+    level_nodes = std::max(level_nodes, P.level_off[l + 1] - P.level_off[l]);
+  }
+  {
+    const size_t need = (size_t)(front[0] + front[1]) * 8 + (size_t)(P.g_total + P.t_total) * 4 +
+                        (size_t)panel * kDirectPanel * 16;
+    size_t free_b = 0, total_b = 0;
+    CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    if (need > free_b / 4) return;
+  }
+  std::vector<DirectNodeDev> nd;
+  for (auto& n : P.nodes)
+    nd.push_back({n.m, n.b, n.ids, n.u, (int)n.front, n.panel, n.ms, n.bs, (long long)n.g,
+                  (long long)n.t});
+  std::vector<std::vector<int>> kids(P.nodes.size());
+  for (int i = 1; i < (int)P.nodes.size(); ++i) kids[P.nodes[i].parent].push_back(i);
+  int dev = 0, sms = 0;
+  CUDA_CHECK(cudaGetDevice(&dev));
+  CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  std::vector<int2> tasks;
+  std::vector<int4> lists;
+  levels_.resize(nl);
+  int want = 1;
+  size_t vec = 0;
+  for (int l = 0; l < nl; ++l) {
+    Level& L = levels_[l];
+    const int n0 = P.level_off[l], n1 = P.level_off[l + 1];
+    L.nodes = n1 - n0;
+    L.ent0 = P.ent_off[l];
+    L.ent1 = P.ent_off[l + 1];
+    L.diag0 = P.diag_off[l];
+    L.diag1 = P.diag_off[l + 1];
+    L.front = P.level_front[l];
+    DirectStage fw, bw;
+    fw.task = (int)tasks.size();
+    for (int i = n0; i < n1; ++i) {
+      const DirectNode& n = P.nodes[i];
+      // A front without a boundary still condenses its own residual.
+      for (int c = 0; c < std::max(n.b, 1); c += 32) tasks.push_back(make_int2(i, c));
+      fw.rows_max = std::max(fw.rows_max, n.m);
+      bw.rows_max = std::max(bw.rows_max, n.m + n.b);
+      L.steps = std::max(L.steps, div_up(n.m, kDirectPanel));
+    }
+    fw.tasks = (int)tasks.size() - fw.task;
+    bw.task = (int)tasks.size();
+    for (int i = n0; i < n1; ++i)
+      for (int c = 0; c < P.nodes[i].m; c += 32) tasks.push_back(make_int2(i, c));
+    bw.tasks = (int)tasks.size() - bw.task;
+    for (DirectStage* s : {&fw, &bw}) {
+      s->warps = group_warps(s->tasks, s->rows_max, sms);
+      const int groups = kWarps / s->warps;
+      vec = std::max(vec, (size_t)groups * s->rows_max);
+      if (l > 0 || s == &bw) want = std::max(want, div_up(s->tasks, groups));
+    }
+    args_.fwd[l] = fw;
+    args_.bwd[l] = bw;
+    L.panel_task = (int)lists.size();
+    for (int i = n0; i < n1; ++i) {
+      const DirectNode& n = P.nodes[i];
+      if (n.m == 0) continue;
+      for (int c = 0; c < n.m + n.b; c += kDirectTile)
+        lists.push_back(make_int4(i, c, i - n0, 0));
+    }
+    L.panel_tasks = (int)lists.size() - L.panel_task;
+    L.tile = (int)lists.size();
+    for (int i = n0; i < n1; ++i) {
+      const DirectNode& n = P.nodes[i];
+      if (n.m == 0) continue;
+      const int k = div_up(n.m + n.b, kDirectTile);
+      for (int x = 0; x < k; ++x)
+        for (int y = x; y < k; ++y) lists.push_back(make_int4(i, x, y, i - n0));
+    }
+    L.tiles = (int)lists.size() - L.tile;
+    for (int s = 0; s < 4; ++s) {
+      L.add[s] = (int)lists.size();
+      for (int i = n0; i < n1; ++i) {
+        if (s >= (int)kids[i].size()) continue;
+        const int k = div_up(P.nodes[kids[i][s]].b, kDirectTile);
+        for (int x = 0; x < k; ++x)
+          for (int y = x; y < k; ++y) lists.push_back(make_int4(kids[i][s], i, x, y));
+      }
+      L.adds[s] = (int)lists.size() - L.add[s];
+    }
+    L.store = (int)lists.size();
+    for (int i = n0; i < n1; ++i) {
+      const DirectNode& n = P.nodes[i];
+      for (int x = 0; x < div_up(n.m, 32); ++x)
+        for (int y = x; y < div_up(n.m + n.b, 32); ++y) lists.push_back(make_int4(i, x, y, 0));
+    }
+    L.stores = (int)lists.size() - L.store;
+  }
+  smem_ = (vec + (size_t)kWarps * 32) * sizeof(float4);
+  const int most = direct_max_blocks(smem_);
+  if (most == 0) return;
+  blocks_ = std::min(want, most);
+  try {
+    upload(P, nd, tasks, lists, front, panel, level_nodes, S.nv, st);
+  } catch (const CudaError&) {
+    // Other worlds took the memory meanwhile: the CG needs none of this.
+    cudaGetLastError();
+    release();
+    return;
+  }
+  args_.nv = S.nv;
+  args_.levels = nl;
+  args_.nodes = nodes_.p;
+  args_.ids = ids_.p;
+  args_.gat_off = gat_off_.p;
+  args_.gat = gat_.p;
+  args_.tasks = tasks_.p;
+  args_.G = G_.p;
+  args_.T = T_.p;
+  args_.u = u_.p;
+  args_.f = f_.p;
+  args_.r = r_.p;
+  args_.dx = dx_.p;
+  args_.xn = xn_.p;
+  args_.partials = partials_.p;
+  args_.barrier = barrier_.p;
+  args_.state = state_.p;
+  usable_ = true;
+}
+
+void DirectSystem::release() {
+  nodes_.reset();
+  for (DevBuf<int>* b : {&ids_, &gat_off_, &gat_, &cmap_, &ent_src_, &ent_dst_, &diag_id_,
+                         &diag_dst_, &state_})
+    b->reset();
+  tasks_.reset();
+  lists_.reset();
+  for (DevBuf<double>* b : {&fronts_[0], &fronts_[1], &V_, &W_, &P_, &partials_}) b->reset();
+  for (DevBuf<float>* b : {&G_, &T_}) b->reset();
+  for (DevBuf<float4>* b : {&u_, &f_, &r_, &dx_, &xn_}) b->reset();
+  barrier_.reset();
+}
+
+void DirectSystem::upload(DirectPlan& P, const std::vector<DirectNodeDev>& nd,
+                          const std::vector<int2>& tasks, const std::vector<int4>& lists,
+                          const int64_t (&front)[2], int panel, int level_nodes, int nv,
+                          cudaStream_t st) {
+  nodes_.upload(nd, st);
+  ids_.upload(P.ids, st);
+  gat_off_.upload(P.gat_off, st);
+  gat_.upload(P.gat, st);
+  if (P.cmap.empty()) P.cmap.push_back(0);
+  cmap_.upload(P.cmap, st);
+  ent_src_.upload(P.ent_src, st);
+  ent_dst_.upload(P.ent_dst, st);
+  diag_id_.upload(P.diag_id, st);
+  diag_dst_.upload(P.diag_dst, st);
+  tasks_.upload(tasks, st);
+  lists_.upload(lists, st);
+  fronts_[0].alloc(std::max<int64_t>(front[0], 1));
+  fronts_[1].alloc(std::max<int64_t>(front[1], 1));
+  V_.alloc((size_t)panel * kDirectPanel);
+  W_.alloc((size_t)panel * kDirectPanel);
+  P_.alloc((size_t)level_nodes * kDirectPanel * kDirectPanel);
+  G_.alloc(std::max<int64_t>(P.g_total, 1));
+  T_.alloc(P.t_total);
+  u_.alloc(std::max(P.u_total, 1));
+  for (DevBuf<float4>* b : {&f_, &r_, &dx_, &xn_}) b->alloc(nv);
+  partials_.alloc(2 * (size_t)blocks_);
+  barrier_.alloc(2);
+  state_.alloc(2);
+  state_.zero(st);
+}
+
+void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* skip,
+                             cudaStream_t st) {
+  DirectFactorArgs a;
+  a.nodes = nodes_.p;
+  a.ids = ids_.p;
+  a.cmap = cmap_.p;
+  a.ent_src = ent_src_.p;
+  a.ent_dst = ent_dst_.p;
+  a.diag_id = diag_id_.p;
+  a.diag_dst = diag_dst_.p;
+  a.Lvals = Lvals;
+  a.dyn = dyn;
+  a.V = V_.p;
+  a.W = W_.p;
+  a.P = P_.p;
+  a.G = G_.p;
+  a.T = T_.p;
+  a.state = state_.p;
+  a.skip = skip;
+  launch_direct_begin(state_.p, skip, st);
+  for (int l = (int)levels_.size() - 1; l >= 0; --l) {
+    const Level& L = levels_[l];
+    a.F = fronts_[l & 1].p;
+    a.Fc = fronts_[(l + 1) & 1].p;
+    CUDA_CHECK(cudaMemsetAsync(a.F, 0, (size_t)L.front * sizeof(double), st));
+    launch_direct_fill(a, L.ent0, L.ent1, L.diag0, L.diag1, st);
+    for (int s = 0; s < 4; ++s)
+      launch_direct_add(a, nodes_.p, lists_.p + L.add[s], L.adds[s], st);
+    for (int k = 0; k < L.steps; ++k) {
+      launch_direct_panel(a, lists_.p + L.panel_task, L.panel_tasks, k, st);
+      launch_direct_update(a, lists_.p + L.tile, L.tiles, k, st);
+    }
+    launch_direct_store(a, lists_.p + L.store, L.stores, st);
+  }
+}
+
+void DirectSystem::solve(const CgArgs& cg, cudaStream_t st) {
+  DirectArgs a = args_;
+  a.nslices = cg.nslices;
+  a.sl_ptr = cg.sl_ptr;
+  a.sl_w = cg.sl_w;
+  a.ent = cg.ent;
+  a.Ldiag = cg.Ldiag;
+  a.dyn = cg.dyn;
+  a.b = cg.b;
+  a.x = cg.x;
+  a.fail = cg.fail;
+  a.skip = cg.skip;
+  a.rel_tol_dev = cg.rel_tol_dev;
+  a.rel_tol = cg.rel_tol;
+  a.abs_tol = cg.abs_tol;
+  a.barrier_spin_limit = cg.barrier_spin_limit;
+  launch_direct_solve(a, blocks_, smem_, st);
+}
+
+}  // namespace silkb

@@ -448,6 +448,7 @@ __device__ __forceinline__ void mark_fail(const CgArgs& a) {
 template <class Barrier>
 __device__ __forceinline__ void cg_body(const CgArgs& a, Barrier& bar, float* sm_all) {
   if (a.skip && *a.skip) return;  // the ADMM solve already ended (every block alike)
+  if (a.solved && *a.solved) return;
   double* part = a.partials + 4 * blockIdx.x;
   CgTrace tr(a.trace, 0);
   // r = b - A x.
@@ -847,6 +848,7 @@ __device__ __forceinline__ float3 res_row_tmem(const ResShared& s, const float4*
 template <class Barrier>
 __device__ void res_body(const CgArgs& a, Barrier& bar, ResShared& s) {
   if (a.skip && *a.skip) return;  // the ADMM solve already ended (every block alike)
+  if (a.solved && *a.solved) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k = blockIdx.x;
   const int nblocks = gridDim.x;
@@ -1538,6 +1540,7 @@ __device__ __forceinline__ float3 dsm_row_tmem(unsigned taddr, int rw, int tm_rw
 template <int F>
 __global__ void __launch_bounds__(32 * F, 1) cg_dsm_cluster_kernel(CgArgs a) {
   if (a.skip && *a.skip) return;  // the ADMM solve already ended (every CTA alike)
+  if (a.solved && *a.solved) return;
   constexpr int W = F, T = 32 * F;
   extern __shared__ __align__(16) unsigned char dsm_smem[];
   DsmShared<W>& s = *reinterpret_cast<DsmShared<W>*>(dsm_smem);

@@ -101,6 +101,9 @@ struct CgArgs {
   // not null.
   const int* skip = nullptr;
   const float* rel_tol_dev = nullptr;
+  // Set when the direct solve queued before this launch met the tolerance:
+  // the kernel returns at entry (null = no direct solve).
+  const int* solved = nullptr;
   long long barrier_spin_limit = 0;  // > 0: grid-barrier polls before giving up
   int withhold_block = -1;      // >= 0: that block skips its barrier arrivals (tests)
   // Cluster form with redundant coarse levels (cg_dsm_cluster_kernel): fine

@@ -10,6 +10,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "collision.cuh"
+#include "direct_system.hpp"
 #include "world.hpp"
 #include "learned.cuh"
 
@@ -27,6 +28,13 @@ struct NvtxRange {
 }  // namespace
 
 namespace {
+
+// ADMM iteration from which a solve's systems go to the direct form, and with
+// them those of every later ADMM solve of the step.  A factorisation costs
+// about four CG solves (0.9 ms against 0.24 at 6,400 vertices, 6.5 against
+// 1.7 at 100K), so short solves stay with the CG; one that has come this far
+// is likely to take as many iterations again.
+constexpr int kDirectFrom = 16;
 
 std::vector<float4> to_float4(const std::vector<float>& v3, const std::vector<int>& perm) {
   int n = (int)perm.size();
@@ -640,6 +648,7 @@ void World::build_cloth_device(Cloth& c) {
   ClothDev& d = c.dev;
   cudaStream_t st = stream;
   int nv = S.nv;
+  d.direct.reset();
   // Sliced ELL of the off-diagonal part, 32 rows per slice.
   int nsl = div_up(nv, 32);
   std::vector<int> sl_ptr(nsl + 1, 0), sl_w(nsl, 0);
@@ -1033,7 +1042,7 @@ float World::warm_sigma() const {
   return std::max(s, 1e-12f);
 }
 
-void World::cg_solve(Cloth& c, float rel_tol, bool first, cudaStream_t st) {
+void World::cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStream_t st) {
   CgArgs a = c.dev.cg;
   a.first_solve = first ? 1 : 0;
   if (first && has_model && opt.learned_warm_start) {
@@ -1063,9 +1072,6 @@ void World::cg_solve(Cloth& c, float rel_tol, bool first, cudaStream_t st) {
   a.withhold_block = opt.debug_withhold_block - 1;
   const bool dsm = c.dev.dsm_ctas > 0;
   const bool resident = !dsm && c.dev.res_grid != 0;
-  // Counted by admm_solve for the iterations that ran.
-  if (dsm || resident) solve_resident_ += 1;
-  if (dsm) solve_cluster_ += 1;
   a.skip = cg_skip_;
   a.rel_tol_dev = cg_skip_ ? &ctl.p->next_rel_tol : nullptr;
   auto launch = [&]() {
@@ -1076,7 +1082,16 @@ void World::cg_solve(Cloth& c, float rel_tol, bool first, cudaStream_t st) {
     else
       launch_cg(a, c.dev.cg_grid, st);
   };
-  if (opt.profile) {
+  // The direct solve takes the system where it meets the tolerance; the CG
+  // behind it returns at entry then, and solves from the same start if not.
+  if (direct && c.dev.direct->usable()) {
+    auto* ev = opt.profile ? next_event_pair(events_other, events_other_used) : nullptr;
+    if (ev) CUDA_CHECK(cudaEventRecord(ev->first, st));
+    c.dev.direct->solve(a, st);
+    a.solved = c.dev.direct->solved();
+    launch();
+    if (ev) CUDA_CHECK(cudaEventRecord(ev->second, st));
+  } else if (opt.profile) {
     auto* ev = next_event_pair(events, events_used);
     CUDA_CHECK(cudaEventRecord(ev->first, st));
     launch();
@@ -1235,7 +1250,6 @@ bool World::admm_solve() {
     const int*& p;
     ~SkipReset() { p = nullptr; }
   } skip_reset{cg_skip_};
-  solve_resident_ = solve_cluster_ = 0;
   const int prior_iterations = stats.admm_iterations;
   int enqueued = 0;
   int fb = face_step_blocks(nf_total), vb = vertex_step_blocks(nv_total);
@@ -1270,7 +1284,17 @@ bool World::admm_solve() {
     if (!iter_sigma.p) iter_sigma.alloc(1);
   }
   DevBuf<float4>* iter_ring[3] = {&iter_hist0, &iter_hist1, &iter_hist2};
+  bool factored = false;  // the direct factors of this solve's matrix are queued
   for (int it = 0; it < g.max_inner_iteration; ++it) {
+    const bool direct = opt.cg_form == 0 && it > 0 && (step_direct_ || it >= kDirectFrom);
+    // A factorisation costs a few CG solves: not for a solve that has just
+    // ended.
+    if (direct && !factored && it > 1) {
+      CUDA_CHECK(cudaMemcpyAsync(&ctl_host_, ctl.p, sizeof(AdmmControl), cudaMemcpyDeviceToHost,
+                                 st));
+      sync();
+      if (ctl_host_.done) break;
+    }
     if (it != 0 && (iter_model || iter_capture)) {
       // x holds x_(it-1); slots (it-1) % 3 and (it-2) % 3 hold x_(it-2) and
       // x_(it-3) from the previous iterations.
@@ -1320,12 +1344,19 @@ bool World::admm_solve() {
           CUDA_CHECK(cudaStreamWaitEvent(cs, fork_ev_, 0));
         }
         if (it == 1) factorize(c, cs);
-        cg_solve(c, rel, it == 1, cs);
+        if (direct && !factored) {
+          if (!c.dev.direct)
+            c.dev.direct = std::make_shared<DirectSystem>(*c.setup, c.rest, cs);
+          if (c.dev.direct->usable())
+            c.dev.direct->factorize(c.dev.Lvals.p, lhs.p + c.voff, done, cs);
+        }
+        cg_solve(c, rel, it == 1, direct, cs);
         if (cs != st) {
           CUDA_CHECK(cudaEventRecord(cloth_done_[k], cs));
           ++f;
         }
       }
+      factored = direct;
       for (int k : forked) CUDA_CHECK(cudaStreamWaitEvent(st, cloth_done_[k], 0));
       if (it == 1 && (opt.capture_samples & 1) && warm_first_) {
         warm_target(nv_total, x.p, ypred.p, 1.0f / warm_sigma(), warm_tgt.p, st);
@@ -1357,14 +1388,10 @@ bool World::admm_solve() {
     if (ctl_host_.done) break;
   }
   // Iterations that ran: 0 .. the last one finalized (the first has no
-  // finalize); each one from the second on ran one CG solve per cloth.
+  // finalize).
   const int ran = enqueued <= 1 ? enqueued : ctl_host_.iteration + 1;
   stats.admm_iterations += ran;
-  if (enqueued > 1) {
-    const int per_it_res = solve_resident_ / (enqueued - 1), per_it_cl = solve_cluster_ / (enqueued - 1);
-    stats.cg_resident_solves += per_it_res * (ran - 1);
-    stats.cg_cluster_solves += per_it_cl * (ran - 1);
-  }
+  if (ran > kDirectFrom) step_direct_ = true;
   if (ctl_host_.diverged) return false;
   launch_enforce(s, st);
   return true;
@@ -1381,6 +1408,7 @@ silk_status World::solver_step() {
     };
     auto t_step = clk::now();
     stats = silk_step_stats{};
+    step_direct_ = false;
     if (cloths.empty()) {
       last_error = "nothing to solve";
       return SILK_ERR_UNKNOWN;
@@ -1513,6 +1541,9 @@ silk_status World::solver_step() {
       const int* q = &cgs[kCgStats * k];
       stats.cg_iterations += q[0];
       stats.cg_solves += q[1];
+      if (cloths[k]->dev.dsm_ctas > 0) stats.cg_cluster_solves += q[1];
+      if (cloths[k]->dev.dsm_ctas > 0 || cloths[k]->dev.res_grid != 0)
+        stats.cg_resident_solves += q[1];
       stats.cg_first_solve_iterations += q[2];
       stats.learned_starts += q[3];
       stats.extrapolated_starts += q[4];

@@ -16,6 +16,8 @@
 
 namespace silkb {
 
+class DirectSystem;
+
 // Owning device allocation.
 template <class T>
 struct DevBuf {
@@ -117,6 +119,7 @@ struct ClothDev {
   DevBuf<int> dsm_push_off, dsm_push;  // its pushes of fine-level z to other CTAs' halos
   CgArgs cg;
   int cg_grid = 1;
+  std::shared_ptr<DirectSystem> direct;  // built when an ADMM solve first needs it
   double bytes_per_iter_fp32 = 0.0;  // algorithmic DRAM bytes per CG iteration
   double bytes_per_iter_bf16 = 0.0;
 };
@@ -231,7 +234,7 @@ class World {
   DevBuf<AdmmControl> ctl;
   AdmmControl ctl_host_{};          // last control block read by admm_solve
   const int* cg_skip_ = nullptr;    // AdmmControl::done while an ADMM solve is enqueued
-  int solve_resident_ = 0, solve_cluster_ = 0;  // CG launches of the solve, by form
+  bool step_direct_ = false;  // an ADMM solve of this step ran long: direct from the start
   DevBuf<int> cg_fail;  // kFail* bits: a bounded device wait gave up, a bank pivot failed
   // Learned warm start: model, step history, features and training samples.
   DevBuf<float> mlp_params, mlp_out, warm_feat, warm_tgt;
@@ -277,7 +280,7 @@ class World {
   void build_resident_layout(Cloth& c);
   void upload_pins();
   void factorize(Cloth& c, cudaStream_t st);
-  void cg_solve(Cloth& c, float rel_tol, bool first, cudaStream_t st);
+  void cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStream_t st);
   void ensure_cloth_streams(size_t n);
   std::vector<cudaStream_t> cloth_streams_;  // per-cloth CG streams (multi-cloth worlds)
   std::vector<cudaEvent_t> cloth_done_;

@@ -1,0 +1,95 @@
+"""The direct form of long ADMM solves (nested-dissection factors applied with
+refinement) against the CG it replaces."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from silk_physics_b200 import native as N
+from silk_physics_b200 import scenes as S
+
+DIRECT_FROM = 16  # ADMM iteration from which the systems go to the direct form
+
+
+def _strip(nx, ny):
+    V, F = S.grid_sheet(max(nx, ny), side=1.0, jitter=1e-4, seed=1)
+    s = max(nx, ny)
+    keep = [j * s + i for j in range(ny) for i in range(nx)]
+    new = -np.ones(s * s, int)
+    new[keep] = np.arange(len(keep))
+    F = new[F]
+    return V[keep], F[(F >= 0).all(1)].astype(np.int32)
+
+
+def _mesh(kind):
+    if kind == "triangle":
+        return (np.array([[0, 0, 1], [0.02, 0, 1], [0, 0.02, 1]], np.float32),
+                np.array([[0, 1, 2]], np.int32))
+    if kind.startswith("sphere"):
+        return S.icosphere(int(kind[6:]), 0.3)
+    nx, ny = (int(k) for k in kind.split("x"))
+    return _strip(nx, ny)
+
+
+# One front (3 to 256 vertices, both sides of a 64 tile and a 32 panel), two
+# and more levels, leaf sizes of both ranges, a long strip and closed surfaces
+# (no boundary to the separators' advantage).
+@pytest.mark.parametrize("kind", ["triangle", "4x8", "5x13", "16x16", "16x17", "40x40", "7x200",
+                                  "sphere3", "sphere4", "150x150"])
+def test_direct_form_matches_cg(kind):
+    """Forty ADMM iterations per step, three steps: the default form solves
+    the systems from DIRECT_FROM on directly, form 1 by CG throughout, both to
+    a relative residual of 1e-6.  Forty unconverged iterations amplify what
+    either leaves, so the yardstick is the CG itself: the direct form must be
+    within three times the CG's own distance (at least 5e-6 m, the FP32 bound
+    of the well-conditioned parity test) of the CG solved to 1e-8."""
+    V, F = _mesh(kind)
+    out = []
+    for form, tol in ((0, 1e-6), (1, 1e-6), (1, 1e-8)):
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(max_inner_iteration=40, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=tol, cg_form=form))
+        r, h = w.add_cloth(N.ClothConfig(elastic_stiffness=10.0, bending_stiffness=1e-4,
+                                         density=5.0, damping=0.01),
+                           N.CollisionConfig(is_collision_on=False, is_self_collision_on=False),
+                           V, F, [0])
+        assert r, r.to_string()
+        for _ in range(3):
+            r = w.solver_step()
+            assert r, r.to_string()
+            st = w.step_stats()
+            assert st.admm_iterations == 40
+            assert st.cg_solves == (DIRECT_FROM - 1 if form == 0 else 39)
+        x = np.zeros(V.size, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append(x.astype(np.float64))
+    err, own = np.abs(out[0] - out[2]).max(), np.abs(out[1] - out[2]).max()
+    print(f"{kind}: direct {err:.2e}, CG {own:.2e} from the CG at 1e-8")
+    assert np.isfinite(out[0]).all()
+    assert err <= max(3.0 * own, 5e-6)
+
+
+def test_direct_form_leaves_what_it_cannot_meet_to_the_cg():
+    """A tolerance that no refinement reaches (1e-30): no direct solve
+    may be taken, every system is solved by the CG from its own start, and
+    the step gives the CG form's bits."""
+    V, F = S.grid_sheet(24, jitter=1e-4, seed=3)
+    out = []
+    for form in (0, 3):
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(max_inner_iteration=24, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0, linear_solver_abs_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-30, cg_form=form,
+                                                    cg_max_iter=40))
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+            is_collision_on=False, is_self_collision_on=False), V, F, S.top_corner_pins(24))
+        assert r
+        assert w.solver_step()
+        assert w.step_stats().cg_solves == 23
+        x = np.zeros(V.size, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append(x)
+    np.testing.assert_array_equal(out[0], out[1])
