@@ -375,15 +375,16 @@ __device__ __forceinline__ float dot3(float3 a, float3 b) {
 // Gauss-Seidel (gs_accum, gs_move).
 __device__ __forceinline__ float3 coulomb_project(float3 us, float3 n, float mu) {
   const float un = fmaf(us.z, n.z, fmaf(us.y, n.y, us.x * n.x));
-  if (un >= 0.0f) return us;
   const float3 ut = make_float3(fmaf(-un, n.x, us.x), fmaf(-un, n.y, us.y), fmaf(-un, n.z, us.z));
   const float ut2 = fmaf(ut.z, ut.z, fmaf(ut.y, ut.y, ut.x * ut.x));
   const float radius = -mu * un;
-  return ut2 <= radius * radius ? make_float3(0.f, 0.f, 0.f)
-                                : sc3(fmaf(-radius, rsqrtf(ut2), 1.0f), ut);
+  // Selected, not branched: the lanes of a warp take all three cases.
+  const float3 slid = sc3(fmaf(-radius, rsqrtf(ut2), 1.0f), ut);
+  const float3 in = ut2 <= radius * radius ? make_float3(0.f, 0.f, 0.f) : slid;
+  return un >= 0.0f ? us : in;
 }
 
-// Contact Gauss-Seidel updates shared by its three forms (identical bits):
+// Contact Gauss-Seidel updates shared by its two forms (identical bits):
 // u += c x (relative position of a contact) and x += g d (a vertex moved by
 // its share g of a correction d).
 __device__ __forceinline__ float3 gs_accum(float3 u, float c, float4 x) {
@@ -1313,18 +1314,11 @@ __global__ void contact_gs_kernel(const ContactDev* contacts, const int* groups,
     }
 }
 
-// Single-block form of contact_gs_kernel.  The contacts are stored in colour
-// order with their cloth vertices renamed to compact slots (the vertices any
-// contact touches), so a colour phase reads contact q = group_off[c] + thread
-// directly and the positions of all touched vertices stay in shared memory for
-// the whole solve; colour phases are separated by __syncthreads and the next
-// phase's contact and correction are loaded while the current one is
-// processed.  The corrections are gathered into colour order at the start and
-// scattered back at the end.  Each contact goes through the same operations
-// in the same order as in contact_gs_kernel (contacts of one colour touch
-// disjoint vertices), so both forms give identical results.
-constexpr int kGsBlockThreads = 1024;
+// Contact records of the single-block form, in colour order with their cloth
+// vertices renamed to compact slots (the vertices any contact touches).
+constexpr int kGsFlowWarps = 12;
 constexpr size_t kGsBlockSmemMax = 226 * 1024;
+constexpr int kGsWaitSpins = 1 << 20;  // polls before a contact gives up
 
 struct GsContact {
   int slot[4];  // compact vertex slot, -1 kinematic
@@ -1371,7 +1365,7 @@ __global__ void gs_gather_kernel(const ContactDev* __restrict__ c, const int* __
   g.affine = k.affine;
   // Bit 31 of ci: the contact's cloth vertices are pairwise distinct, so the
   // positions gathered for its relative position are still current when it
-  // is applied (the pipelined kernel then skips re-reading them).
+  // is applied (the kernel then skips re-reading them).
   bool distinct = true;
   for (int a = 0; a < 4; ++a)
     for (int b = a + 1; b < 4; ++b)
@@ -1393,14 +1387,6 @@ __global__ void gs_inc_keys_kernel(const GsContact* __restrict__ cc, int total, 
   key[e] = k.gamma[s] != 0.0f && k.slot[s] >= 0 ? k.slot[s] : 0x7fffffff;
   val[e] = e;
 }
-// The sorted entries as (contact position, share bits) pairs.
-__global__ void gs_vent_kernel(const GsContact* __restrict__ cc, const int* __restrict__ code,
-                               int n, int2* __restrict__ vent) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const int c = code[e], q = c >> 2;
-  vent[e] = make_int2(q, __float_as_int(cc[q].gamma[c & 3]));
-}
 // voff[i] = first entry of slot i in the sorted keys, for i <= nslots (info[4]).
 __global__ void gs_voff_kernel(const int* __restrict__ sorted, int n, const int* info, int nv,
                                int* voff) {
@@ -1415,174 +1401,135 @@ __global__ void gs_voff_kernel(const int* __restrict__ sorted, int n, const int*
   voff[i] = lo;
 }
 
-__global__ void __launch_bounds__(kGsBlockThreads) contact_gs_block_kernel(
-    const GsContact* __restrict__ cc, const int* __restrict__ group_off, int ncolors, int total,
-    float4* __restrict__ corr, float4* __restrict__ ccorr, const int* __restrict__ vlist,
-    int nslots, float4* __restrict__ p, const int* __restrict__ skip) {
-  if (skip && *skip) return;  // the ADMM solve already ended
-  extern __shared__ float4 sp[];
-  const int t = threadIdx.x;
-  for (int i = t; i < nslots; i += blockDim.x) sp[i] = p[vlist[i]];
-  for (int q = t; q < total; q += blockDim.x) ccorr[q] = corr[cc[q].ci & 0x7fffffff];
-  __syncthreads();
-  // Warm start with the saved corrections.
-  for (int col = 0; col < ncolors; ++col) {
-    int q = group_off[col] + t;
-    if (q < group_off[col + 1]) {
-      const GsContact& k = cc[q];
-      float4 r = ccorr[q];
-      for (int s = 0; s < 4; ++s) {
-        if (k.gamma[s] == 0.0f) continue;
-        float4 x = sp[k.slot[s]];
-        float g = k.gamma[s];
-        sp[k.slot[s]] = gs_move(x, g, make_float3(r.x, r.y, r.z));
-      }
-    }
-    __syncthreads();
+// The sorted entries as (contact position, share bits) pairs, and per entry
+// of the contacts (4 q + s) its place among its slot's entries (low half; the
+// first of them for a vertex the contact names twice) and their number (high
+// half), 0 for a vertex the contact does not move.  A vertex has at most four
+// entries per colour and 1,024 colours, so both fit 16 bits.
+__global__ void gs_vent_kernel(const GsContact* __restrict__ cc, const int* __restrict__ code,
+                               const int* __restrict__ sorted, const int* __restrict__ voff,
+                               int n, int2* __restrict__ vent, unsigned* __restrict__ place) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int c = code[e], q = c >> 2;
+  vent[e] = make_int2(q, __float_as_int(cc[q].gamma[c & 3]));
+  const int slot = sorted[e];
+  unsigned at = 0u;
+  if (slot != 0x7fffffff) {
+    const int e0 = voff[slot];
+    int first = e;
+    while (first > e0 && (code[first - 1] >> 2) == q) --first;
+    at = (unsigned)(first - e0) | ((unsigned)(voff[slot + 1] - e0) << 16);
   }
-  // A thread always takes the same contact of a colour, so the correction it
-  // prefetches was last written by itself.
-  auto fetch = [&](int col, int& q, GsContact& k, float4& o) {
-    q = group_off[col] + t;
-    if (q < group_off[col + 1]) {
-      k = cc[q];
-      o = ccorr[q];
-    } else {
-      q = -1;
-    }
+  place[c] = at;
+}
+// Records of the single-block form as six arrays of 16 bytes, so that a
+// warp's loads are contiguous: slots and places (16 bits each); entry counts,
+// contact index (bit 31: distinct slots) and friction; coefficients; shares;
+// normal and the affine part.
+__global__ void gs_rec_kernel(const GsContact* __restrict__ cc, const unsigned* __restrict__ place,
+                              int total, const int* info, int4* __restrict__ rec) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= total) return;
+  const GsContact k = cc[q];
+  const int zero = info[4];  // the slot that reads as zero
+  unsigned sl[4], rk[4], dg[4];
+  for (int s = 0; s < 4; ++s) {
+    const unsigned at = place[4 * q + s];
+    sl[s] = (unsigned)(k.slot[s] >= 0 ? k.slot[s] : zero) & 0xffffu;
+    rk[s] = at & 0xffffu;
+    dg[s] = at >> 16;
+  }
+  rec[q] = make_int4((int)(sl[0] | sl[1] << 16), (int)(sl[2] | sl[3] << 16),
+                     (int)(rk[0] | rk[1] << 16), (int)(rk[2] | rk[3] << 16));
+  rec[total + q] = make_int4((int)(dg[0] | dg[1] << 16), (int)(dg[2] | dg[3] << 16), k.ci,
+                             __float_as_int(k.friction));
+  auto pack = [](float a, float b, float c, float d) {
+    return make_int4(__float_as_int(a), __float_as_int(b), __float_as_int(c), __float_as_int(d));
   };
-  const int phases = kGsSweeps * ncolors;
-  int qn = -1;
-  GsContact k;
-  float4 on = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (phases > 0) fetch(0, qn, k, on);
-  for (int ph = 0; ph < phases; ++ph) {
-    const int cur = qn;
-    const GsContact kc = k;
-    const float4 o = on;
-    if (ph + 1 < phases) fetch((ph + 1) % ncolors, qn, k, on);
-    if (cur >= 0) {
-      float3 u = kc.affine;
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const float4 x = kc.slot[s] >= 0 ? sp[kc.slot[s]] : make_float4(0.f, 0.f, 0.f, 0.f);
-        u = gs_accum(u, kc.coef[s], x);
-      }
-      float3 old = make_float3(o.x, o.y, o.z);
-      float3 us = sub3(u, old);
-      float3 unew = coulomb_project(us, kc.normal, kc.friction);
-      float3 du = sub3(unew, u);
-      float3 nc = add3(old, du);
-      ccorr[cur] = make_float4(nc.x, nc.y, nc.z, 0.f);
-      if (qn == cur) on = make_float4(nc.x, nc.y, nc.z, 0.f);  // one colour
-      for (int s = 0; s < 4; ++s) {
-        if (kc.gamma[s] == 0.0f) continue;
-        float4 x = sp[kc.slot[s]];
-        float g = kc.gamma[s];
-        sp[kc.slot[s]] = gs_move(x, g, make_float3(du.x, du.y, du.z));
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = t; q < total; q += blockDim.x) corr[cc[q].ci & 0x7fffffff] = ccorr[q];
-  for (int i = t; i < nslots; i += blockDim.x) p[vlist[i]] = sp[i];
+  rec[2 * total + q] = pack(k.coef[0], k.coef[1], k.coef[2], k.coef[3]);
+  rec[3 * total + q] = pack(k.gamma[0], k.gamma[1], k.gamma[2], k.gamma[3]);
+  rec[4 * total + q] = pack(k.normal.x, k.normal.y, k.normal.z, k.affine.x);
+  rec[5 * total + q] = pack(k.affine.y, k.affine.z, 0.f, 0.f);
 }
 
-// Pipelined single-block form: the contact records of the next ns colour
-// phases (ns = 4 staging stages, or 2 or 1 when 4 do not fit shared memory)
-// arrive in shared memory by bulk copies (one per colour: its
-// records are contiguous in colour order) while the current phase is
-// processed, each completing on its stage's mbarrier; the corrections and
-// colour offsets stay in shared memory for the whole call, so a phase never
-// waits on a global load.  Same per-contact operations as contact_gs_kernel.
-constexpr int kGsStages = 4;  // most stages (2 or 1 when 4 do not fit shared memory)
-static_assert(sizeof(GsContact) % 16 == 0, "bulk copies move whole 16-byte units");
-constexpr int kGsWaitSpins = 1 << 20;  // mbarrier polls before a phase gives up
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
+// Contact positions of the single-block form in shared memory: (x, y, z) and,
+// in the last word, how many corrections the vertex has received.  Written
+// and read as one 128-bit scalar, so a reader sees both or neither.
+__device__ __forceinline__ float4 gs_load(unsigned addr) {
+  unsigned long long lo, hi;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      "{\n .reg .b128 v;\n ld.relaxed.cta.shared.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}\n"
+      : "=l"(lo), "=l"(hi)
+      : "r"(addr)
       : "memory");
-  return ok != 0;
+  return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)),
+                     __uint_as_float((unsigned)hi), __uint_as_float((unsigned)(hi >> 32)));
 }
-// Bounded wait for phase `parity` of an mbarrier: false if it did not complete.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  for (int spin = 0; spin < kGsWaitSpins; ++spin)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-// Bulk copy global -> this CTA's shared memory, completing on `bar`.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes,
-                                              uint64_t* bar) {
+__device__ __forceinline__ void gs_store(unsigned addr, float4 x) {
+  const unsigned long long lo =
+      ((unsigned long long)__float_as_uint(x.y) << 32) | __float_as_uint(x.x);
+  const unsigned long long hi =
+      ((unsigned long long)__float_as_uint(x.w) << 32) | __float_as_uint(x.z);
   asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-      ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      "{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.cta.shared.b128 [%0], v;\n}\n" ::"r"(
+          addr),
+      "l"(lo), "l"(hi)
       : "memory");
 }
 
-struct GsPipeLayout {
-  size_t sp, sc, go, stage, bytes;
-};
-__host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
-__host__ __device__ inline GsPipeLayout gs_pipe_layout(int nslots, int total, int ncolors,
-                                                       int threads, int stages) {
-  GsPipeLayout L;
-  L.sp = 0;
-  // Two extra position slots: nslots reads as zero (kinematic vertices),
-  // nslots + 1 takes the stores of zero-share vertices.
-  L.sc = align16(L.sp + (size_t)(nslots + 2) * sizeof(float4));
-  L.go = align16(L.sc + (size_t)total * sizeof(float4));
-  L.stage = align16(L.go + (size_t)(ncolors + 1) * sizeof(int));
-  L.bytes = L.stage + (size_t)stages * threads * sizeof(GsContact);
-  return L;
-}
-
-__global__ void __launch_bounds__(kGsBlockThreads) contact_gs_pipe_kernel(
-    const GsContact* __restrict__ cc, const int* __restrict__ group_off, int ncolors, int total,
-    float4* __restrict__ corr, const int* __restrict__ vlist, int nslots, float4* __restrict__ p,
-    int* __restrict__ fail, const int* __restrict__ skip, const int* __restrict__ voff,
-    const int2* __restrict__ vent, int ns_log) {
+// Single-block form of contact_gs_kernel, ordered by data instead of by
+// barriers.  The positions of every touched vertex stay in shared memory and
+// carry a count of the corrections they have received; in each sweep a
+// contact runs as soon as its movable vertices have received exactly the
+// corrections of the contacts before it in colour order.  Every vertex thus
+// receives the same moves in the same order as in the colour phases of the
+// grid form (bit-identical results), but a contact waits for its own
+// predecessors only and not for the slowest contact of every colour.
+//
+// Warp w takes the batches of 32 contacts w, w + W, ... of the colour order,
+// sweep after sweep, one contact per lane; a lane polls the vertices whose
+// count is not yet right and keeps the positions of the others.  The earliest
+// unfinished contact of all has no unfinished predecessor and is in the batch
+// at the head of its warp's list, so some contact can always run; the polls
+// are bounded all the same (kGsWaitSpins, then kFailContactWait and the
+// positions are left untouched).  Records stream from L2 one batch ahead into
+// registers.
+//
+// Bound by the latency of one contact (poll, projection, store: ~570 cycles)
+// times the longest chain of contacts through shared vertices, about the
+// number of colours per sweep.  With colour phases (a block barrier per
+// colour, records staged by bulk copies) most of a phase was the barrier's
+// wait for the slowest warp: Gauss-Seidel per step 42 ms for the settling
+// 80 x 80 scene (2,536 contacts, 22 colours) and 132 ms for a 41 x 41 sheet at
+// first contact (519 contacts, 75 colours), against 31 and 75 ms here.  Four
+// lanes per contact (one per vertex, positions exchanged by shuffles) took 48
+// and 92 ms.
+template <bool kCorrShared>
+__global__ void __launch_bounds__(kGsFlowWarps * 32) contact_gs_flow_kernel(
+    const int4* __restrict__ rec, int total, float4* __restrict__ corr,
+    float4* __restrict__ ccorr, const int* __restrict__ vlist, int nslots,
+    float4* __restrict__ p, int* __restrict__ fail, const int* __restrict__ skip,
+    const int* __restrict__ voff, const int2* __restrict__ vent) {
   if (skip && *skip) return;  // the ADMM solve already ended
   extern __shared__ __align__(16) unsigned char gs_raw[];
-  __shared__ __align__(8) uint64_t bars[kGsStages];
-  const int ns = 1 << ns_log, nmask = ns - 1;  // staging stages: 1, 2 or 4
-  const GsPipeLayout L = gs_pipe_layout(nslots, total, ncolors, blockDim.x, ns);
-  float4* sp = reinterpret_cast<float4*>(gs_raw + L.sp);
-  float4* sc = reinterpret_cast<float4*>(gs_raw + L.sc);
-  int* sgo = reinterpret_cast<int*>(gs_raw + L.go);
-  GsContact* stage = reinterpret_cast<GsContact*>(gs_raw + L.stage);
-  const int t = threadIdx.x, nt = blockDim.x;
-  for (int i = t; i < nslots; i += nt) sp[i] = p[vlist[i]];
-  if (t < 2) sp[nslots + t] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int zslot = nslots, tslot = nslots + 1;
-  for (int q = t; q < total; q += nt) sc[q] = corr[cc[q].ci & 0x7fffffff];
-  for (int c = t; c <= ncolors; c += nt) sgo[c] = group_off[c];
+  __shared__ int lost;
+  float4* sp = reinterpret_cast<float4*>(gs_raw);
+  // One extra position slot that reads as zero (kinematic vertices).
+  float4* sc = kCorrShared ? sp + nslots + 1 : ccorr;
+  const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warps = nt >> 5;
+  if (t == 0) {
+    lost = 0;
+    sp[nslots] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int q = t; q < total; q += nt) sc[q] = corr[rec[total + q].z & 0x7fffffff];
   __syncthreads();
   // Warm start with the saved corrections: each slot applies those of its
   // contacts in colour order (its entries of the slot incidence), the same
-  // moves in the same order as colour phases would, without their barriers.
-  // A slot's entries (at most 8 per load round) are loaded together.
+  // moves in the same order as colour phases would.  A slot's entries (at
+  // most 8 per load round) are loaded together.
   for (int i = t; i < nslots; i += nt) {
-    float4 x = sp[i];
+    float4 x = p[vlist[i]];
     const int e1 = voff[i + 1];
     for (int e0 = voff[i]; e0 < e1; e0 += 8) {
       int2 en[8];
@@ -1595,115 +1542,118 @@ __global__ void __launch_bounds__(kGsBlockThreads) contact_gs_pipe_kernel(
         x = gs_move(x, __int_as_float(en[k].y), make_float3(r.x, r.y, r.z));
       }
     }
+    x.w = __int_as_float(0);
     sp[i] = x;
   }
   __syncthreads();
-  const int phases = kGsSweeps * ncolors;
-  // The copies are issued by the block's last thread: its warp holds no
-  // contact in most colours, so the issue stays off the contacts' path.
-  const int producer = nt - 1;
-  if (t == producer) {
-    for (int s = 0; s < ns; ++s) mbar_init(&bars[s], 1);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  }
-  __syncthreads();
-  // Copy the records of phase ph's colour into stage ph % ns.  A thread reads
-  // its record of phase ph at the end of phase ph - 1, before that phase's
-  // block barrier, so at phase ph the stage of phase ph is free again and
-  // receives the records of phase ph + ns.
-  auto issue = [&](int ph, int col) {
-    if (t != producer || ph >= phases) return;
-    uint64_t* bar = &bars[ph & nmask];
-    const unsigned bytes = (unsigned)((sgo[col + 1] - sgo[col]) * (int)sizeof(GsContact));
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    if (bytes) {
-      mbar_arrive_expect(bar, bytes);
-      bulk_copy_g2s(stage + (size_t)(ph & nmask) * nt, cc + sgo[col], bytes, bar);
-    } else {
-      mbar_arrive(bar);
-    }
-  };
-  int col_issue = 0;
-#pragma unroll
-  for (int s = 0; s < ns; ++s) {
-    issue(s, col_issue);
-    col_issue = col_issue + 1 == ncolors ? 0 : col_issue + 1;
-  }
-  // Registers carry the record and the correction of the phase about to run;
-  // they are loaded before the previous phase's barrier, so their latency
-  // overlaps the barrier.  A thread always takes the same contact of a
-  // colour, so the correction it loads was last written by itself (with one
-  // colour, in the phase just run, earlier in this thread's program order).
-  GsContact kn;
+  const unsigned base = (unsigned)__cvta_generic_to_shared(sp);
+  const int nb = (total + 31) / 32;
+  int4 r0, r1, r2, r3, r4, r5;
   float4 on = make_float4(0.f, 0.f, 0.f, 0.f);
-  int qn = -1;
-  bool lost = false;  // a copy this thread waited for did not land in time
-  auto fetch = [&](int ph, int col) {
-    const bool landed = mbar_wait(&bars[ph & nmask], (unsigned)(ph >> ns_log) & 1u);
-    qn = sgo[col] + t;
-    if (landed && qn < sgo[col + 1]) {
-      kn = stage[(size_t)(ph & nmask) * nt + t];
-      on = sc[qn];
-    } else {
-      qn = -1;
-    }
-    lost = lost || !landed;
+  auto fetch = [&](int b) {
+    const int q = min(b * 32 + lane, total - 1);
+    r0 = rec[q];
+    r1 = rec[total + q];
+    r2 = rec[2 * total + q];
+    r3 = rec[3 * total + q];
+    r4 = rec[4 * total + q];
+    r5 = rec[5 * total + q];
+    return q;
   };
-  int col = 0;
-  if (phases > 0) fetch(0, 0);
-  __syncthreads();  // every thread has read stage 0 before phase 0 refills it
-  int ph = 0;
-  for (; ph < phases; ++ph) {
-    issue(ph + ns, col_issue);
-    col_issue = col_issue + 1 == ncolors ? 0 : col_issue + 1;
-    const int cur = qn;
-    const GsContact kc = kn;
-    const float4 o = on;
-    col = col + 1 == ncolors ? 0 : col + 1;
-    if (cur >= 0) {
-      // All four positions read at once, without branches (a kinematic
-      // vertex reads the zero slot: u gains c * 0).
-      float3 u = kc.affine;
-      float4 xs[4];
-#pragma unroll
-      for (int s = 0; s < 4; ++s) xs[s] = sp[kc.slot[s] >= 0 ? kc.slot[s] : zslot];
-#pragma unroll
-      for (int s = 0; s < 4; ++s) u = gs_accum(u, kc.coef[s], xs[s]);
-      float3 old = make_float3(o.x, o.y, o.z);
-      float3 us = sub3(u, old);
-      float3 unew = coulomb_project(us, kc.normal, kc.friction);
-      float3 du = sub3(unew, u);
-      float3 nc = add3(old, du);
-      sc[cur] = make_float4(nc.x, nc.y, nc.z, 0.f);
-      const bool distinct = kc.ci < 0;
-      // Zero-share vertices (kinematic, pinned) store into the scratch slot.
+  int b = t >> 5, sweep = 0;
+  if (b < nb) on = sc[fetch(b)];
+  bool go = b < nb;
+  while (go && sweep < kGsSweeps) {
+    const int q = b * 32 + lane;
+    unsigned addr[4];
+    int want[4];
+    unsigned moves = 0u;
+    {
+      const int sl[2] = {r0.x, r0.y}, rk[2] = {r0.z, r0.w}, dg[2] = {r1.x, r1.y};
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
-        const int sl = kc.gamma[s] != 0.0f && kc.slot[s] >= 0 ? kc.slot[s] : tslot;
-        const float4 x = distinct ? xs[s] : sp[sl];
-        sp[sl] = gs_move(x, kc.gamma[s], du);
+        const int sh = 16 * (s & 1);
+        addr[s] = base + 16u * (((unsigned)sl[s >> 1] >> sh) & 0xffffu);
+        const int deg = (int)(((unsigned)dg[s >> 1] >> sh) & 0xffffu);
+        moves |= deg != 0 ? 1u << s : 0u;
+        want[s] = (int)(((unsigned)rk[s >> 1] >> sh) & 0xffffu) + sweep * deg;
       }
     }
-    if (ph + 1 < phases) fetch(ph + 1, col);
-    // The block barrier that orders the colours also agrees on a lost copy,
-    // so every thread leaves the loop at the same phase.
-    if (__syncthreads_or(lost)) break;
-  }
-  if (ph < phases) {
-    // A copy did not land in time: wait (bounded) for the copies still in
-    // flight, report the failure (the step then returns
-    // IterativeSolveFail) and leave the positions untouched.
-    if (t == producer) {
-      // Phase ph's copy completed before phase ph - 1's barrier; ph + 1 ..
-      // ph + ns may still be in flight.
-      for (int q = ph + 1; q <= ph + ns && q < phases; ++q)
-        mbar_wait(&bars[q & nmask], (unsigned)(q >> ns_log) & 1u);
-      if (fail) atomicOr(fail, kFailContactWait);
+    const bool distinct = r1.z < 0;
+    const float mu = __int_as_float(r1.w);
+    const float coef[4] = {__int_as_float(r2.x), __int_as_float(r2.y), __int_as_float(r2.z),
+                           __int_as_float(r2.w)};
+    const float gam[4] = {__int_as_float(r3.x), __int_as_float(r3.y), __int_as_float(r3.z),
+                          __int_as_float(r3.w)};
+    const float3 nrm =
+        make_float3(__int_as_float(r4.x), __int_as_float(r4.y), __int_as_float(r4.z));
+    const float3 aff =
+        make_float3(__int_as_float(r4.w), __int_as_float(r5.x), __int_as_float(r5.y));
+    const float3 old = make_float3(on.x, on.y, on.z);
+    // The next batch of this warp, in registers before this one has to wait.
+    int bn = b + warps, sn = sweep;
+    if (bn >= nb) {
+      bn = t >> 5;
+      ++sn;
     }
+    if (sn < kGsSweeps) {
+      const int qn = fetch(bn);
+      if (bn != b) on = sc[qn];
+    }
+    float4 xs[4];
+    unsigned need = q < total ? 15u : 0u;  // vertices still to be waited for
+    bool pending = q < total;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) xs[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int spin = 0; __any_sync(0xffffffffu, pending); ++spin) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        if (need & (1u << s)) xs[s] = gs_load(addr[s]);
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        if (!(moves & (1u << s)) || __float_as_int(xs[s].w) == want[s]) need &= ~(1u << s);
+      if (pending && need == 0u) {
+        float3 u = aff;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) u = gs_accum(u, coef[s], xs[s]);
+        const float3 us = sub3(u, old);
+        const float3 unew = coulomb_project(us, nrm, mu);
+        const float3 du = sub3(unew, u);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          // A vertex that the contact names twice takes both moves in turn.
+          if (!distinct && (moves & (1u << s))) xs[s] = gs_load(addr[s]);
+          float4 y = gs_move(xs[s], gam[s], du);
+          y.w = __int_as_float(__float_as_int(xs[s].w) + 1);
+          if (moves & (1u << s)) gs_store(addr[s], y);
+        }
+        const float3 nc = add3(old, du);
+        const float4 c = make_float4(nc.x, nc.y, nc.z, 0.f);
+        sc[q] = c;
+        if (bn == b) on = c;  // this warp's only batch
+        pending = false;
+      }
+      // Every lane of the warp takes the same decision.
+      if ((spin & 255) == 255 &&
+          __any_sync(0xffffffffu, spin >= kGsWaitSpins || *(volatile int*)&lost != 0)) {
+        *(volatile int*)&lost = 1;
+        go = false;
+        break;
+      }
+    }
+    b = bn;
+    sweep = sn;
+  }
+  __syncthreads();
+  if (lost) {
+    if (t == 0 && fail) atomicOr(fail, kFailContactWait);
     return;
   }
-  for (int q = t; q < total; q += nt) corr[cc[q].ci & 0x7fffffff] = sc[q];
-  for (int i = t; i < nslots; i += nt) p[vlist[i]] = sp[i];
+  for (int q = t; q < total; q += nt) corr[rec[total + q].z & 0x7fffffff] = sc[q];
+  for (int i = t; i < nslots; i += nt) {
+    const float4 x = sp[i];
+    p[vlist[i]] = make_float4(x.x, x.y, x.z, 0.f);
+  }
 }
 
 // Canonical contact key (contact_constraints.cu:24-47).
@@ -1826,6 +1776,8 @@ struct CollisionImpl {
   // slot's in colour order; gs_voff[slot] = its first entry).
   DevBuf<int> gs_ikey, gs_ival, gs_ikey_s, gs_vinc, gs_voff;
   DevBuf<int2> gs_vent;  // sorted entries as (contact position, share bits)
+  DevBuf<unsigned> gs_place;  // per entry: place among its vertex's and their number
+  DevBuf<int4> gs_rec;        // the single-block form's records
   DevBuf<char> sort_temp;
   DevBuf<int> pick_d;  // DCD records picked as new contacts (grow-only)
   DevBuf<unsigned> gs_barrier;
@@ -2403,7 +2355,7 @@ int CollisionSystem::append_active(float time, float dact) {
     gs_gather_kernel<<<div_up(total, kCollThreads), kCollThreads, 0, st>>>(
         I.contacts.p, I.groups.p, total, I.gs_slot.p, I.gs_cc.p);
     SILK_LAUNCHED();
-    // Slot incidence in colour order for the pipelined form's warm start.
+    // Slot incidence in colour order for the single-block form.
     const int ne = 4 * total;
     I.gs_ikey.alloc(ne);
     I.gs_ival.alloc(ne);
@@ -2424,7 +2376,13 @@ int CollisionSystem::append_active(float time, float dact) {
                                                         I.gs_voff.p);
     SILK_LAUNCHED();
     I.gs_vent.alloc(ne);
-    gs_vent_kernel<<<div_up(ne, 256), 256, 0, st>>>(I.gs_cc.p, I.gs_vinc.p, ne, I.gs_vent.p);
+    I.gs_place.alloc(ne);
+    gs_vent_kernel<<<div_up(ne, 256), 256, 0, st>>>(I.gs_cc.p, I.gs_vinc.p, I.gs_ikey_s.p,
+                                                    I.gs_voff.p, ne, I.gs_vent.p, I.gs_place.p);
+    SILK_LAUNCHED();
+    I.gs_rec.alloc(6 * (size_t)total);
+    gs_rec_kernel<<<div_up(total, 256), 256, 0, st>>>(I.gs_cc.p, I.gs_place.p, total,
+                                                      I.col_info.p, I.gs_rec.p);
     SILK_LAUNCHED();
     I.gs_ready = true;
   }
@@ -2444,44 +2402,30 @@ void CollisionSystem::contact_solve_launch() {
   CollisionImpl& I = *impl_;
   if (I.n_contacts == 0) return;
   cudaStream_t st = w_.stream;
-  const size_t smem = (size_t)I.gs_nslots * sizeof(float4);
-  if (I.gs_ready && w_.opt.contact_gs_form != 1 && I.max_group <= kGsBlockThreads &&
-      smem <= kGsBlockSmemMax) {
+  // Single-block form while the touched vertices' positions fit the block's
+  // shared memory, with the corrections too where they also fit.
+  const size_t pos = (size_t)(I.gs_nslots + 1) * sizeof(float4);
+  const size_t both = pos + (size_t)I.n_contacts * sizeof(float4);
+  if (I.gs_ready && w_.opt.contact_gs_form != 1 && pos <= kGsBlockSmemMax) {
     static const bool attr = [] {
-      CUDA_CHECK(cudaFuncSetAttribute(contact_gs_block_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kGsBlockSmemMax));
+      for (auto* k : {contact_gs_flow_kernel<true>, contact_gs_flow_kernel<false>})
+        CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kGsBlockSmemMax));
       return true;
     }();
     (void)attr;
-    // Only as many warps as the largest colour needs: every colour phase ends
-    // in a block barrier, whose cost grows with the number of warps.
-    const int threads = std::max(32, div_up(I.max_group, 32) * 32);
-    // Four staging stages where they fit, else two, else one (the copy for a
-    // colour is then issued 4, 2 or 1 phases ahead).
-    int ns_log = 2;
-    GsPipeLayout L = gs_pipe_layout(I.gs_nslots, I.n_contacts, I.n_colors, threads, 4);
-    while (L.bytes > kGsBlockSmemMax && ns_log > 0) {
-      --ns_log;
-      L = gs_pipe_layout(I.gs_nslots, I.n_contacts, I.n_colors, threads, 1 << ns_log);
-    }
-    if (L.bytes <= kGsBlockSmemMax) {
-      static const bool pattr = [] {
-        CUDA_CHECK(cudaFuncSetAttribute(contact_gs_pipe_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kGsBlockSmemMax));
-        return true;
-      }();
-      (void)pattr;
-      contact_gs_pipe_kernel<<<1, threads, L.bytes, st>>>(
-          I.gs_cc.p, I.group_off.p, I.n_colors, I.n_contacts, I.corr.p, I.gs_vlist.p,
-          I.gs_nslots, w_.contact_p.p, w_.cg_fail.p, gs_skip_, I.gs_voff.p, I.gs_vent.p, ns_log);
-      SILK_LAUNCHED();
-      return;
-    }
-    contact_gs_block_kernel<<<1, threads, smem, st>>>(
-        I.gs_cc.p, I.group_off.p, I.n_colors, I.n_contacts, I.corr.p, I.gs_ccorr.p,
-        I.gs_vlist.p, I.gs_nslots, w_.contact_p.p, gs_skip_);
+    const bool shared = both <= kGsBlockSmemMax;
+    // About six batches a warp: fewer leave warps polling beside the ones
+    // that work, more put contacts that could run behind ones that wait
+    // (ms of Gauss-Seidel per step with 2, 4, 8, 12 and 16 warps: 64, 40, 32,
+    // 31 and 32 for 2,536 contacts, 75, 75, 78, 80 and 84 for 519).
+    const int batches = div_up(I.n_contacts, 32);
+    const int threads =
+        32 * std::min(batches, std::min(kGsFlowWarps, std::max(2, div_up(batches, 6))));
+    auto* kernel = shared ? contact_gs_flow_kernel<true> : contact_gs_flow_kernel<false>;
+    kernel<<<1, threads, shared ? both : pos, st>>>(
+        I.gs_rec.p, I.n_contacts, I.corr.p, I.gs_ccorr.p, I.gs_vlist.p,
+        I.gs_nslots, w_.contact_p.p, w_.cg_fail.p, gs_skip_, I.gs_voff.p, I.gs_vent.p);
     SILK_LAUNCHED();
     return;
   }

@@ -12,7 +12,7 @@ namespace silkb {
 // convergence test and reported as IterativeSolveFail.
 constexpr int kFailBarrier = 1;   // a grid-barrier wait of a CG kernel gave up
 constexpr int kFailMasPivot = 2;  // a MAS bank had a zero or non-finite pivot
-constexpr int kFailContactWait = 4;  // a contact Gauss-Seidel copy did not land in time
+constexpr int kFailContactWait = 4;  // a contact Gauss-Seidel wait gave up
 
 constexpr int kPacked = BANK * (BANK + 1) / 2;  // 528 packed upper entries
 

@@ -1484,7 +1484,7 @@ silk_status World::solver_step() {
         CUDA_CHECK(cudaMemcpy(&f, cg_fail.p, sizeof(int), cudaMemcpyDeviceToHost));
         last_error = (f & kFailMasPivot) ? "MAS bank inverse failed: zero or non-finite pivot"
                      : (f & kFailBarrier) ? "CG barrier wait gave up"
-                     : (f & kFailContactWait) ? "contact Gauss-Seidel copy wait gave up"
+                     : (f & kFailContactWait) ? "contact Gauss-Seidel wait gave up"
                      : (f & kFailMlpWait) ? "learned warm start tensor-core wait gave up"
                                           : "solver diverged";
         if (f) cg_fail.zero(st);

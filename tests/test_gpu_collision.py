@@ -298,3 +298,39 @@ def test_gs_forms_identical():
     assert max(out[0][1]) > 0
     assert out[0][1] == out[1][1]
     np.testing.assert_array_equal(out[0][0], out[1][0])
+
+
+# Cloth side, obstacle side, gap in paddings: one batch of contacts on one
+# warp; several batches with a remainder; more than the block's shared memory
+# holds corrections for (226 KB / 16 B = 14,464 positions and corrections).
+@pytest.mark.parametrize("s,so,few,many", [(2, 2, 1, 31), (12, 9, 100, 2000),
+                                           (78, 78, 14464, 1 << 20)])
+def test_gs_single_block_sizes_identical(s, so, few, many):
+    """A sheet within contact distance of a flat obstacle, two ADMM
+    iterations: the single-block Gauss-Seidel (contacts ordered by their
+    vertices' counts) and the grid form (ordered by colour barriers) move
+    every vertex alike, bit for bit."""
+    out = []
+    for form in (0, 1):
+        V, F = S.grid_sheet(s, side=0.5 * (s - 1) / 77, z=1.0, jitter=1e-6, seed=4)
+        OV, OF = S.grid_sheet(so, side=0.52 * (s - 1) / 77, z=0.0)
+        OV[:, 2] = V[:, 2].min() - 0.3 * 0.05 * 0.5 / 77
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(acceleration_z=-9.81, max_inner_iteration=3,
+                                                  max_outer_iteration=1))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5,
+                                                    contact_gs_form=form))
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(is_self_collision_on=False), V, F,
+                           [])
+        r2, _ = w.add_obstacle(N.CollisionConfig(), OV, OF)
+        assert r and r2
+        r = w.solver_step()
+        assert r, r.to_string()
+        x = np.zeros(V.size, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append((x, w.step_stats().contacts))
+    print(f"{s} x {s} over {so} x {so}: {out[0][1]} contacts")
+    assert few <= out[0][1] <= many
+    assert out[0][1] == out[1][1]
+    np.testing.assert_array_equal(out[0][0], out[1][0])
