@@ -248,86 +248,100 @@ __global__ void tree_up_kernel(float4* nodes, int L, int k) {
   }
 }
 
+// One query primitive per thread against the tree of another primitive set
+// (oibvh.cuh:418-516).  mode: 0 PT inter, 1 PT self, 2 EE inter, 3 EE self.
 // Candidate record: x = primitive of A, y = primitive of B,
 // z = (kind << 16) | slot A, w = slot B.  kind 0: A triangle / B point;
 // kind 1: A edge / B edge.
-struct Emitter {
-  int4* out;
-  int cap;
-  int* counter;
-  int4 buf[8];
-  int n = 0;
-  __device__ void flush() {
-    if (n == 0) return;
-    int at = atomicAdd(counter, n);
-    for (int i = 0; i < n; ++i)
-      if (at + i < cap) out[at + i] = buf[i];
-    n = 0;
-  }
-  __device__ void push(int4 r) {
-    buf[n++] = r;
-    if (n == 8) flush();
-  }
-};
-
-// One query primitive per thread against the tree of another primitive set
-// (oibvh.cuh:418-516).  mode: 0 PT inter, 1 PT self, 2 EE inter, 3 EE self.
-__global__ void traverse_kernel(const ObjDev* objs, int tslot, int qslot, int mode,
-                                int4* out, int cap, int* counter) {
+//
+// A node's two children are neighbours in memory and tested together: the
+// loads of both boxes are in flight at once and only overlapping children
+// are visited (a leaf's box is its primitive's).  A self query of edges skips
+// subtrees whose leaves all come at or after its own (each pair once).  The
+// hits of a query are kept in a short list; a warp's lists are appended with
+// one atomic at the end, since one per query on the shared counter had been
+// the limit: 473 us a launch on the 100K-vertex sheet.
+constexpr int kTraverseList = 16;
+__global__ void __launch_bounds__(kCollThreads) traverse_kernel(const ObjDev* objs, int tslot,
+                                                                int qslot, int mode, int4* out,
+                                                                int cap, int* counter) {
   const ObjDev& T = objs[tslot];
   const ObjDev& Q = objs[qslot];
-  bool pt = mode < 2;
-  bool self = (mode & 1) != 0;
-  int nq = pt ? Q.nv : Q.ne;
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  Emitter em{out, cap, counter};
+  const bool pt = mode < 2;
+  const bool self = (mode & 1) != 0;
+  const int nq = pt ? Q.nv : Q.ne;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  int list[kTraverseList];
+  int held = 0, qprim = 0;
+  auto record = [&](int tprim) {
+    if (!pt && self && qprim < tprim)
+      return make_int4(qprim, tprim, (1 << 16) | tslot, qslot);
+    return make_int4(tprim, qprim, (pt ? 0 : 1 << 16) | tslot, qslot);
+  };
+  auto write = [&](int at) {
+    for (int i = 0; i < held; ++i)
+      if (at + i < cap) out[at + i] = record(list[i]);
+    held = 0;
+  };
   if (q < nq) {
-    int qprim = (mode == 3) ? Q.edge_order[q] : q;
-    Box qb = load_box(pt ? Q.pt_bb : Q.edge_bb, qprim);
-    int D = pt ? T.tri_D : T.edge_D;
-    int n = pt ? T.nf : T.ne;
+    qprim = (mode == 3) ? Q.edge_order[q] : q;
+    const Box qb = load_box(pt ? Q.pt_bb : Q.edge_bb, qprim);
+    const int D = pt ? T.tri_D : T.edge_D;
+    const int n = pt ? T.nf : T.ne;
     const float4* nodes = pt ? T.tri_nodes : T.edge_nodes;
     const int* order = pt ? T.tri_order : T.edge_order;
-    const float4* prim_bb = pt ? T.tri_bb : T.edge_bb;
-    int Pn = 1 << D;
-    unsigned stack[64];
+    const int2 qe = pt ? make_int2(qprim, -1) : Q.E[qprim];
+    const float qmass = pt ? Q.inv_mass[qprim] : 0.0f;
+    unsigned stack[32];
     int sp = 0;
-    if (n > 0) stack[sp++] = 0u;
+    if (n > 0 && overlap(qb, load_box(nodes, 0))) stack[sp++] = 0u;
     while (sp > 0) {
-      unsigned node = stack[--sp];
-      int depth = 31 - __clz((int)(node + 1u));
-      if (!overlap(qb, load_box(nodes, (int)node))) continue;
+      const unsigned node = stack[--sp];
+      const int depth = 31 - __clz((int)(node + 1u));
       if (depth == D) {
-        int leaf = (int)node - (Pn - 1);
-        if (leaf >= n) continue;
-        if (mode == 3 && !(leaf < q)) continue;
-        int tprim = order[leaf];
-        if (!overlap(qb, load_box(prim_bb, tprim))) continue;
+        const int leaf = (int)(node + 1u) - (1 << D);
+        if (leaf >= n || (mode == 3 && leaf >= q)) continue;
+        const int tprim = order[leaf];
         if (pt) {
-          int4 f = T.F[tprim];
-          float s = Q.inv_mass[qprim] + T.inv_mass[f.x] + T.inv_mass[f.y] + T.inv_mass[f.z];
-          if (s == 0.0f) continue;
+          const int4 f = T.F[tprim];
+          if (qmass + T.inv_mass[f.x] + T.inv_mass[f.y] + T.inv_mass[f.z] == 0.0f) continue;
           if (self && (f.x == qprim || f.y == qprim || f.z == qprim)) continue;
-          em.push(make_int4(tprim, qprim, (0 << 16) | tslot, qslot));
         } else {
-          int2 a = T.E[tprim], b = Q.E[qprim];
-          float s = T.inv_mass[a.x] + T.inv_mass[a.y] + Q.inv_mass[b.x] + Q.inv_mass[b.y];
-          if (s == 0.0f) continue;
-          if (self && (a.x == b.x || a.x == b.y || a.y == b.x || a.y == b.y)) continue;
-          if (self) {
-            int lo = tprim < qprim ? tprim : qprim, hi = tprim < qprim ? qprim : tprim;
-            em.push(make_int4(lo, hi, (1 << 16) | tslot, qslot));
-          } else {
-            em.push(make_int4(tprim, qprim, (1 << 16) | tslot, qslot));
-          }
+          const int2 a = T.E[tprim];
+          if (T.inv_mass[a.x] + T.inv_mass[a.y] + Q.inv_mass[qe.x] + Q.inv_mass[qe.y] == 0.0f)
+            continue;
+          if (self && (a.x == qe.x || a.x == qe.y || a.y == qe.x || a.y == qe.y)) continue;
         }
-      } else {
-        stack[sp++] = 2u * node + 2u;
-        stack[sp++] = 2u * node + 1u;
+        list[held++] = tprim;
+        if (held == kTraverseList) write(atomicAdd(counter, kTraverseList));
+        continue;
       }
+      const float4* c = nodes + 2 * (size_t)(2u * node + 1u);
+      const float4 l0 = c[0], l1 = c[1], r0 = c[2], r1 = c[3];
+      Box lb, rb;
+      lb.mn = make_float3(l0.x, l0.y, l0.z);
+      lb.mx = make_float3(l1.x, l1.y, l1.z);
+      rb.mn = make_float3(r0.x, r0.y, r0.z);
+      rb.mx = make_float3(r1.x, r1.y, r1.z);
+      // First leaf below the right child.
+      const unsigned right = 2u * node + 2u;
+      const long long first = (long long)(right + 1u - (2u << depth)) << (D - depth - 1);
+      if (overlap(qb, rb) && (mode != 3 || first < q)) stack[sp++] = right;
+      if (overlap(qb, lb)) stack[sp++] = right - 1u;
     }
   }
-  em.flush();
+  // Append the warp's lists behind one another.
+  const int lane = threadIdx.x & 31;
+  int sum = held;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += v;
+  }
+  int base = 0;
+  if (lane == 31 && sum > 0) base = atomicAdd(counter, sum);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  write(base + sum - held);
 }
 
 // ---------------------------------------------------------------------------
