@@ -11,7 +11,7 @@ namespace silkb {
 // Device copy of one front (see DirectNode).
 struct DirectNodeDev {
   int m, b, ids, u, front, panel, ms, bs;
-  long long g, t;
+  long long g, t, gd;
 };
 
 // Work of one tree level in the application kernel: tasks (node, first
@@ -36,8 +36,7 @@ struct DirectArgs {
   float4* x = nullptr;
   const DirectNodeDev* nodes = nullptr;
   const int* ids = nullptr;
-  const int* gat_off = nullptr;
-  const int* gat = nullptr;
+  const int4* gat = nullptr;  // per entry of ids: updates summed into it (-1 none)
   const int2* tasks = nullptr;
   DirectStage fwd[kDirectMaxLevels], bwd[kDirectMaxLevels];
   const float* G = nullptr;
@@ -48,7 +47,7 @@ struct DirectArgs {
   float4* dx = nullptr;   // correction of the current application
   float4* xn = nullptr;   // x plus the corrections so far
   double* partials = nullptr;
-  unsigned* barrier = nullptr;  // [count, err]
+  unsigned* barrier = nullptr;  // [count, err, blocks that left]
   int* state = nullptr;  // [0] factorisation failed, [1] this solve met its tolerance
   int* fail = nullptr;   // kFail* word of the solver
   const int* skip = nullptr;
@@ -73,6 +72,7 @@ struct DirectFactorArgs {
   double* V = nullptr;        // panel scratch: old and eliminated pivot rows
   double* W = nullptr;
   double* P = nullptr;        // inverted pivot blocks
+  double* Gd = nullptr;       // G of this level in FP64
   float* G = nullptr;
   float* T = nullptr;
   int* state = nullptr;
@@ -82,7 +82,7 @@ struct DirectFactorArgs {
 // Blocks of the application kernel that are resident at once on this device
 // with `smem` bytes of dynamic shared memory (0: not launchable).
 int direct_max_blocks(size_t smem);
-void launch_direct_begin(int* state, const int* skip, cudaStream_t st);
+void launch_direct_begin(int* state, unsigned* barrier, const int* skip, cudaStream_t st);
 void launch_direct_fill(const DirectFactorArgs& a, int ent0, int ent1, int diag0, int diag1,
                         cudaStream_t st);
 // tiles: (child node, tile row, tile column) of one child slot.
@@ -93,6 +93,8 @@ void launch_direct_panel(const DirectFactorArgs& a, const int4* tasks, int n, in
 void launch_direct_update(const DirectFactorArgs& a, const int4* tiles, int n, int step,
                           cudaStream_t st);
 void launch_direct_store(const DirectFactorArgs& a, const int4* tiles, int n, cudaStream_t st);
+void launch_direct_products(const DirectFactorArgs& a, const int4* gtiles, int ng,
+                            const int4* stiles, int ns, cudaStream_t st);
 void launch_direct_solve(const DirectArgs& a, int blocks, size_t smem, cudaStream_t st);
 
 }  // namespace silkb

@@ -1,5 +1,6 @@
 // Host side of the direct ADMM solve (see direct_system.hpp).
 #include <algorithm>
+#include <type_traits>
 
 #include "direct_system.hpp"
 
@@ -38,22 +39,32 @@ DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
   if (nl > kDirectMaxLevels) return;
   int64_t front[2] = {0, 0};
   int panel = 0, level_nodes = 0;
+  int64_t gd = 1;  // most entries of a level's G
+  std::vector<int64_t> node_gd(P.nodes.size(), 0);
   for (int l = 0; l < nl; ++l) {
+    int64_t at = 0;
+    for (int i = P.level_off[l]; i < P.level_off[l + 1]; ++i) {
+      node_gd[i] = at;
+      at += (int64_t)P.nodes[i].m * P.nodes[i].b;
+    }
+    gd = std::max(gd, at);
     front[l & 1] = std::max(front[l & 1], P.level_front[l]);
     panel = std::max(panel, P.level_panel[l]);
     level_nodes = std::max(level_nodes, P.level_off[l + 1] - P.level_off[l]);
   }
   {
-    const size_t need = (size_t)(front[0] + front[1]) * 8 + (size_t)(P.g_total + P.t_total) * 4 +
+    const size_t need = (size_t)(front[0] + front[1] + gd) * 8 + (size_t)(P.g_total + P.t_total) * 4 +
                         (size_t)panel * kDirectPanel * 16;
     size_t free_b = 0, total_b = 0;
     CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
     if (need > free_b / 4) return;
   }
   std::vector<DirectNodeDev> nd;
-  for (auto& n : P.nodes)
+  for (size_t i = 0; i < P.nodes.size(); ++i) {
+    const DirectNode& n = P.nodes[i];
     nd.push_back({n.m, n.b, n.ids, n.u, (int)n.front, n.panel, n.ms, n.bs, (long long)n.g,
-                  (long long)n.t});
+                  (long long)n.t, (long long)node_gd[i]});
+  }
   std::vector<std::vector<int>> kids(P.nodes.size());
   for (int i = 1; i < (int)P.nodes.size(); ++i) kids[P.nodes[i].parent].push_back(i);
   int dev = 0, sms = 0;
@@ -100,7 +111,7 @@ DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
     for (int i = n0; i < n1; ++i) {
       const DirectNode& n = P.nodes[i];
       if (n.m == 0) continue;
-      for (int c = 0; c < n.m + n.b; c += kDirectTile)
+      for (int c = 0; c < n.m; c += kDirectTile)
         lists.push_back(make_int4(i, c, i - n0, 0));
     }
     L.panel_tasks = (int)lists.size() - L.panel_task;
@@ -108,7 +119,7 @@ DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
     for (int i = n0; i < n1; ++i) {
       const DirectNode& n = P.nodes[i];
       if (n.m == 0) continue;
-      const int k = div_up(n.m + n.b, kDirectTile);
+      const int k = div_up(n.m, kDirectTile);
       for (int x = 0; x < k; ++x)
         for (int y = x; y < k; ++y) lists.push_back(make_int4(i, x, y, i - n0));
     }
@@ -127,119 +138,148 @@ DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
     for (int i = n0; i < n1; ++i) {
       const DirectNode& n = P.nodes[i];
       for (int x = 0; x < div_up(n.m, 32); ++x)
-        for (int y = x; y < div_up(n.m + n.b, 32); ++y) lists.push_back(make_int4(i, x, y, 0));
+        for (int y = x; y < div_up(n.m, 32); ++y) lists.push_back(make_int4(i, x, y, 0));
     }
     L.stores = (int)lists.size() - L.store;
+    L.product = (int)lists.size();
+    for (int i = n0; i < n1; ++i)
+      for (int x = 0; x < div_up(P.nodes[i].m, kDirectTile); ++x)
+        for (int y = 0; y < div_up(P.nodes[i].b, kDirectTile); ++y)
+          lists.push_back(make_int4(i, x, y, 0));
+    L.products = (int)lists.size() - L.product;
+    L.schur = (int)lists.size();
+    for (int i = n0; i < n1; ++i)
+      for (int x = 0; x < (P.nodes[i].m ? div_up(P.nodes[i].b, kDirectTile) : 0); ++x)
+        for (int y = x; y < div_up(P.nodes[i].b, kDirectTile); ++y)
+          lists.push_back(make_int4(i, x, y, 0));
+    L.schurs = (int)lists.size() - L.schur;
   }
   smem_ = (vec + (size_t)kWarps * 32) * sizeof(float4);
   const int most = direct_max_blocks(smem_);
   if (most == 0) return;
   blocks_ = std::min(want, most);
   try {
-    upload(P, nd, tasks, lists, front, panel, level_nodes, S.nv, st);
+    upload(P, nd, tasks, lists, front, gd, panel, level_nodes, S.nv, st);
   } catch (const CudaError&) {
     // Other worlds took the memory meanwhile: the CG needs none of this.
     cudaGetLastError();
-    release();
+    arena_.reset();
     return;
   }
   args_.nv = S.nv;
   args_.levels = nl;
-  args_.nodes = nodes_.p;
-  args_.ids = ids_.p;
-  args_.gat_off = gat_off_.p;
-  args_.gat = gat_.p;
-  args_.tasks = tasks_.p;
-  args_.G = G_.p;
-  args_.T = T_.p;
-  args_.u = u_.p;
-  args_.f = f_.p;
-  args_.r = r_.p;
-  args_.dx = dx_.p;
-  args_.xn = xn_.p;
-  args_.partials = partials_.p;
-  args_.barrier = barrier_.p;
-  args_.state = state_.p;
+  args_.nodes = nodes_;
+  args_.ids = ids_;
+  args_.gat = reinterpret_cast<const int4*>(gat_);
+  args_.tasks = tasks_;
+  args_.G = G_;
+  args_.T = T_;
+  args_.u = u_;
+  args_.f = f_;
+  args_.r = r_;
+  args_.dx = dx_;
+  args_.xn = xn_;
+  args_.partials = partials_;
+  args_.barrier = barrier_;
+  args_.state = state_;
   usable_ = true;
 }
 
-void DirectSystem::release() {
-  nodes_.reset();
-  for (DevBuf<int>* b : {&ids_, &gat_off_, &gat_, &cmap_, &ent_src_, &ent_dst_, &diag_id_,
-                         &diag_dst_, &state_})
-    b->reset();
-  tasks_.reset();
-  lists_.reset();
-  for (DevBuf<double>* b : {&fronts_[0], &fronts_[1], &V_, &W_, &P_, &partials_}) b->reset();
-  for (DevBuf<float>* b : {&G_, &T_}) b->reset();
-  for (DevBuf<float4>* b : {&u_, &f_, &r_, &dx_, &xn_}) b->reset();
-  barrier_.reset();
-}
-
-void DirectSystem::upload(DirectPlan& P, const std::vector<DirectNodeDev>& nd,
+// One allocation for everything (a first solve otherwise spends longer in
+// two dozen allocations than in its factorisation).
+void DirectSystem::upload(const DirectPlan& P, const std::vector<DirectNodeDev>& nd,
                           const std::vector<int2>& tasks, const std::vector<int4>& lists,
-                          const int64_t (&front)[2], int panel, int level_nodes, int nv,
-                          cudaStream_t st) {
-  nodes_.upload(nd, st);
-  ids_.upload(P.ids, st);
-  gat_off_.upload(P.gat_off, st);
-  gat_.upload(P.gat, st);
-  if (P.cmap.empty()) P.cmap.push_back(0);
-  cmap_.upload(P.cmap, st);
-  ent_src_.upload(P.ent_src, st);
-  ent_dst_.upload(P.ent_dst, st);
-  diag_id_.upload(P.diag_id, st);
-  diag_dst_.upload(P.diag_dst, st);
-  tasks_.upload(tasks, st);
-  lists_.upload(lists, st);
-  fronts_[0].alloc(std::max<int64_t>(front[0], 1));
-  fronts_[1].alloc(std::max<int64_t>(front[1], 1));
-  V_.alloc((size_t)panel * kDirectPanel);
-  W_.alloc((size_t)panel * kDirectPanel);
-  P_.alloc((size_t)level_nodes * kDirectPanel * kDirectPanel);
-  G_.alloc(std::max<int64_t>(P.g_total, 1));
-  T_.alloc(P.t_total);
-  u_.alloc(std::max(P.u_total, 1));
-  for (DevBuf<float4>* b : {&f_, &r_, &dx_, &xn_}) b->alloc(nv);
-  partials_.alloc(2 * (size_t)blocks_);
-  barrier_.alloc(2);
-  state_.alloc(2);
-  state_.zero(st);
+                          const int64_t (&front)[2], int64_t gd, int panel, int level_nodes,
+                          int nv, cudaStream_t st) {
+  size_t need = 0;
+  char* base = nullptr;
+  auto place = [&](auto*& p, size_t count) {
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + need);
+    need += (std::max<size_t>(count, 1) * sizeof(*p) + 255) / 256 * 256;
+  };
+  for (int pass = 0; pass < 2; ++pass) {
+    need = 0;
+    place(nodes_, nd.size());
+    place(ids_, P.ids.size());
+    place(gat_, P.gat.size());
+    place(cmap_, P.cmap.size());
+    place(ent_src_, P.ent_src.size());
+    place(ent_dst_, P.ent_dst.size());
+    place(diag_id_, P.diag_id.size());
+    place(diag_dst_, P.diag_dst.size());
+    place(tasks_, tasks.size());
+    place(lists_, lists.size());
+    place(fronts_[0], front[0]);
+    place(fronts_[1], front[1]);
+    place(V_, (size_t)panel * kDirectPanel);
+    place(W_, (size_t)panel * kDirectPanel);
+    place(P_, (size_t)level_nodes * kDirectPanel * kDirectPanel);
+    place(Gd_, gd);
+    place(G_, P.g_total);
+    place(T_, P.t_total);
+    place(u_, P.u_total);
+    for (float4** v : {&f_, &r_, &dx_, &xn_}) place(*v, nv);
+    place(partials_, 2 * (size_t)blocks_);
+    place(barrier_, 3);
+    place(state_, 2);
+    if (pass == 0) {
+      arena_.alloc(need);
+      base = arena_.p;
+    }
+  }
+  auto copy = [&](auto* to, const auto& from) {
+    if (!from.empty())
+      CUDA_CHECK(cudaMemcpyAsync(to, from.data(), from.size() * sizeof(from[0]),
+                                 cudaMemcpyHostToDevice, st));
+  };
+  copy(nodes_, nd);
+  copy(ids_, P.ids);
+  copy(gat_, P.gat);
+  copy(cmap_, P.cmap);
+  copy(ent_src_, P.ent_src);
+  copy(ent_dst_, P.ent_dst);
+  copy(diag_id_, P.diag_id);
+  copy(diag_dst_, P.diag_dst);
+  copy(tasks_, tasks);
+  copy(lists_, lists);
+  CUDA_CHECK(cudaMemsetAsync(state_, 0, 2 * sizeof(int), st));
 }
 
 void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* skip,
                              cudaStream_t st) {
   DirectFactorArgs a;
-  a.nodes = nodes_.p;
-  a.ids = ids_.p;
-  a.cmap = cmap_.p;
-  a.ent_src = ent_src_.p;
-  a.ent_dst = ent_dst_.p;
-  a.diag_id = diag_id_.p;
-  a.diag_dst = diag_dst_.p;
+  a.nodes = nodes_;
+  a.ids = ids_;
+  a.cmap = cmap_;
+  a.ent_src = ent_src_;
+  a.ent_dst = ent_dst_;
+  a.diag_id = diag_id_;
+  a.diag_dst = diag_dst_;
   a.Lvals = Lvals;
   a.dyn = dyn;
-  a.V = V_.p;
-  a.W = W_.p;
-  a.P = P_.p;
-  a.G = G_.p;
-  a.T = T_.p;
-  a.state = state_.p;
+  a.V = V_;
+  a.W = W_;
+  a.P = P_;
+  a.Gd = Gd_;
+  a.G = G_;
+  a.T = T_;
+  a.state = state_;
   a.skip = skip;
-  launch_direct_begin(state_.p, skip, st);
+  launch_direct_begin(state_, barrier_, skip, st);
   for (int l = (int)levels_.size() - 1; l >= 0; --l) {
     const Level& L = levels_[l];
-    a.F = fronts_[l & 1].p;
-    a.Fc = fronts_[(l + 1) & 1].p;
+    a.F = fronts_[l & 1];
+    a.Fc = fronts_[(l + 1) & 1];
     CUDA_CHECK(cudaMemsetAsync(a.F, 0, (size_t)L.front * sizeof(double), st));
     launch_direct_fill(a, L.ent0, L.ent1, L.diag0, L.diag1, st);
     for (int s = 0; s < 4; ++s)
-      launch_direct_add(a, nodes_.p, lists_.p + L.add[s], L.adds[s], st);
+      launch_direct_add(a, nodes_, lists_ + L.add[s], L.adds[s], st);
     for (int k = 0; k < L.steps; ++k) {
-      launch_direct_panel(a, lists_.p + L.panel_task, L.panel_tasks, k, st);
-      launch_direct_update(a, lists_.p + L.tile, L.tiles, k, st);
+      launch_direct_panel(a, lists_ + L.panel_task, L.panel_tasks, k, st);
+      launch_direct_update(a, lists_ + L.tile, L.tiles, k, st);
     }
-    launch_direct_store(a, lists_.p + L.store, L.stores, st);
+    launch_direct_store(a, lists_ + L.store, L.stores, st);
+    launch_direct_products(a, lists_ + L.product, L.products, lists_ + L.schur, L.schurs, st);
   }
 }
 

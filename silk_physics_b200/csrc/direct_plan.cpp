@@ -240,9 +240,12 @@ bool build_direct_plan(int nv, const std::vector<int>& rows, const std::vector<i
       return false;
     }
   }
-  // Positions of boundaries in the parents' fronts, and what is summed where.
+  // Positions of boundaries in the parents' fronts, and what is summed where:
+  // a front entry receives at most one update of each of its (up to four)
+  // children.
   P.cmap.assign(P.u_total, 0);
-  std::vector<int> place(nv, -1), count(P.ids.size() + 1, 0);
+  P.gat.assign(4 * P.ids.size(), -1);
+  std::vector<int> place(nv, -1);
   std::vector<std::vector<int>> children(P.nodes.size());
   for (int i = 1; i < (int)P.nodes.size(); ++i) children[P.nodes[i].parent].push_back(i);
   for (int i = 0; i < (int)P.nodes.size(); ++i) {
@@ -253,21 +256,11 @@ bool build_direct_plan(int nv, const std::vector<int>& rows, const std::vector<i
       for (int j = 0; j < ch.b; ++j) {
         const int at = place[P.ids[ch.ids + ch.m + j]];
         P.cmap[ch.u + j] = at;
-        ++count[n.ids + at + 1];
+        int* g = &P.gat[4 * (size_t)(n.ids + at)];
+        while (*g >= 0) ++g;
+        *g = ch.u + j;
       }
     }
-  }
-  P.gat_off.assign(P.ids.size() + 1, 0);
-  for (size_t i = 0; i < P.ids.size(); ++i) P.gat_off[i + 1] = P.gat_off[i] + count[i + 1];
-  P.gat.assign(std::max(P.gat_off.back(), 1), 0);
-  {
-    std::vector<int> at(P.gat_off.begin(), P.gat_off.end() - 1);
-    for (int i = 0; i < (int)P.nodes.size(); ++i)
-      for (int c : children[i]) {
-        const DirectNode& ch = P.nodes[c];
-        for (int j = 0; j < ch.b; ++j)
-          P.gat[at[P.nodes[i].ids + P.cmap[ch.u + j]]++] = ch.u + j;
-      }
   }
   P.ent_src.reserve(cols.size() / 2 + nv);
   P.ent_dst.reserve(cols.size() / 2 + nv);

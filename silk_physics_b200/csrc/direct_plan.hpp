@@ -32,7 +32,7 @@ struct DirectPlan {
   std::vector<DirectNode> nodes;        // by level, root first
   std::vector<int> level_off;           // per level: first node (levels + 1 entries)
   std::vector<int> ids;                 // solver vertex ids of every front
-  std::vector<int> gat_off, gat;        // per entry of ids: update entries summed into it
+  std::vector<int> gat;                 // per entry of ids: 4 update entries summed into it (-1 none)
   std::vector<int> cmap;                // per boundary entry: position in the parent's front
   std::vector<int64_t> level_front;     // per level: entries of its front buffer
   std::vector<int> level_panel;         // per level: columns of its panel scratch

@@ -18,7 +18,7 @@ class DirectSystem {
   // Solves into a.x, to the tolerance of the CG solve `cg` stands for.
   void solve(const CgArgs& cg, cudaStream_t st);
   // Set when the last solve met its tolerance (the CG then has nothing to do).
-  const int* solved() const { return state_.p + 1; }
+  const int* solved() const { return state_ + 1; }
 
  private:
   struct Level {
@@ -28,27 +28,31 @@ class DirectSystem {
     int panel_task = 0, panel_tasks = 0;
     int tile = 0, tiles = 0;
     int add[4] = {0, 0, 0, 0}, adds[4] = {0, 0, 0, 0};
-    int store = 0, stores = 0;
+    int store = 0, stores = 0, product = 0, products = 0, schur = 0, schurs = 0;
   };
-  void upload(DirectPlan& P, const std::vector<DirectNodeDev>& nd,
+  void upload(const DirectPlan& P, const std::vector<DirectNodeDev>& nd,
               const std::vector<int2>& tasks, const std::vector<int4>& lists,
-              const int64_t (&front)[2], int panel, int level_nodes, int nv, cudaStream_t st);
-  void release();
+              const int64_t (&front)[2], int64_t gd, int panel, int level_nodes, int nv,
+              cudaStream_t st);
 
   bool usable_ = false;
   int blocks_ = 0;
   size_t smem_ = 0;
   std::vector<Level> levels_;
   DirectArgs args_;
-  DevBuf<DirectNodeDev> nodes_;
-  DevBuf<int> ids_, gat_off_, gat_, cmap_, ent_src_, ent_dst_, diag_id_, diag_dst_;
-  DevBuf<int2> tasks_;
-  DevBuf<int4> lists_;  // panel tasks, update tiles, add tiles and store tiles
-  DevBuf<double> fronts_[2], V_, W_, P_, partials_;
-  DevBuf<float> G_, T_;
-  DevBuf<float4> u_, f_, r_, dx_, xn_;
-  DevBuf<unsigned> barrier_;
-  DevBuf<int> state_;
+  // Everything on the device, in one allocation.
+  DevBuf<char> arena_;
+  DirectNodeDev* nodes_ = nullptr;
+  int *ids_ = nullptr, *gat_ = nullptr, *cmap_ = nullptr, *ent_src_ = nullptr,
+      *ent_dst_ = nullptr, *diag_id_ = nullptr, *diag_dst_ = nullptr;
+  int2* tasks_ = nullptr;
+  int4* lists_ = nullptr;  // panel tasks and the tiles of the other kernels
+  double *fronts_[2] = {nullptr, nullptr}, *V_ = nullptr, *W_ = nullptr, *P_ = nullptr,
+         *Gd_ = nullptr, *partials_ = nullptr;
+  float *G_ = nullptr, *T_ = nullptr;
+  float4 *u_ = nullptr, *f_ = nullptr, *r_ = nullptr, *dx_ = nullptr, *xn_ = nullptr;
+  unsigned* barrier_ = nullptr;
+  int* state_ = nullptr;
 };
 
 }  // namespace silkb
