@@ -433,8 +433,9 @@ silk_status silk_mlp_train(float* params, const float* features, const float* ta
  * allocation outside it can fail or evict), and real-time loops in which
  * cudaMalloc / cudaFree would synchronise the device and stall other
  * streams.  The call performs no cudaMalloc, cudaFree or other allocating
- * routine; its working memory is one static device array of 10,489,088
- * bytes created with the library on each device that loads it.
+ * routine; its working memory is one static device array of 4,194,560
+ * bytes created with the library on each device that loads it, and the
+ * shared memory of its second pass.
  *
  * Buffers x (n x 24 floats), min_separation (n), hit (n), toi (n) and
  * t_upper (n, may be NULL) are device (or managed) memory of the CURRENT

@@ -621,10 +621,8 @@ __device__ bool eval_unit_1d(bool vf, const float3* Pt, float eps, float ms, int
   return true;
 }
 
-__device__ bool eval_box_1d(bool vf, const IBox& b, const CcdCoeff& co, float em,
-                            int dim, bool& in_eps, float& tol) {
-  float c0 = co.c0[dim], c1 = co.c1[dim], c2 = co.c2[dim], c3 = co.c3[dim],
-        c4 = co.c4[dim], c5 = co.c5[dim];
+__device__ bool eval_box_1d(bool vf, const IBox& b, float c0, float c1, float c2, float c3,
+                            float c4, float c5, float em, bool& in_eps, float& tol) {
   float mn[2], mx[2];
   float ts[2] = {b.t0, b.t1};
   for (int k = 0; k < 2; ++k) {
@@ -685,44 +683,26 @@ __device__ float clamp_div(float a, float b, float mx) {
   return smin(a / b, mx);
 }
 
-// Pending boxes of one search: a small per-thread array for the first pass;
-// queries that outgrow it are re-run with a global-memory array of
-// max_iter + 2 entries, the most a search can hold (each evaluation pops one
-// box and pushes at most two, and pushes stop after max_iter evaluations).
 // Pending boxes of a search, in the reference's processing order: smallest
 // t.lower first and, for equal t.lower, the most recently pushed (its
 // std::map of per-t.lower stacks, interval_root_finder.cpp:430-500).  Two
-// stores of that one total order: a sorted array (top = next; an insertion
-// shifts the boxes with smaller t.lower, cheap while the search is shallow)
-// and a binary heap keyed on (t.lower ascending, push sequence descending),
-// O(log n) per operation for deep searches.
+// stores of that one total order.
+
+// One search per thread: a sorted array (top = next; an insertion shifts the
+// boxes with smaller t.lower, cheap while the search is shallow), per thread
+// in the first pass.  Queries that outgrow it are run again with room for
+// max_iter + 2 boxes, the most a search can hold (each evaluation pops one
+// box and pushes at most two, and pushes stop after max_iter evaluations).
 struct DfsStack {
+  static constexpr bool kWarp = false;
   IBox local[kCcdStack];
   IBox* e;
-  int* q = nullptr;  // heap: push sequence of each box
   int cap;
   int n;
-  bool heap = false;
-  int seq = 0;
-  __device__ __forceinline__ bool before(const IBox& a, int qa, const IBox& b, int qb) const {
-    return a.t0 < b.t0 || (a.t0 == b.t0 && qa > qb);
-  }
+  __device__ void reset() { n = 0; }
+  __device__ bool empty() const { return n == 0; }
   __device__ bool push(const IBox& b) {
     if (n >= cap) return false;
-    if (heap) {
-      const int sq = seq++;
-      int i = n++;
-      while (i > 0) {
-        const int p = (i - 1) >> 1;
-        if (!before(b, sq, e[p], q[p])) break;
-        e[i] = e[p];
-        q[i] = q[p];
-        i = p;
-      }
-      e[i] = b;
-      q[i] = sq;
-      return true;
-    }
     int pos = n;
     while (pos > 0 && e[pos - 1].t0 < b.t0) --pos;
     for (int k = n; k > pos; --k) e[k] = e[k - 1];
@@ -730,30 +710,90 @@ struct DfsStack {
     ++n;
     return true;
   }
-  // t.lower of the box pop() would return (n > 0).
-  __device__ __forceinline__ float top_t0() const { return heap ? e[0].t0 : e[n - 1].t0; }
-  __device__ IBox pop() {
-    if (!heap) return e[--n];
-    const IBox top = e[0];
-    --n;
-    if (n > 0) {
-      const IBox last = e[n];
-      const int lq = q[n];
-      int i = 0;
-      for (;;) {
-        const int l = 2 * i + 1;
-        if (l >= n) break;
-        int c = l;
-        if (l + 1 < n && before(e[l + 1], q[l + 1], e[l], q[l])) c = l + 1;
-        if (!before(e[c], q[c], last, lq)) break;
-        e[i] = e[c];
-        q[i] = q[c];
-        i = c;
-      }
-      e[i] = last;
-      q[i] = lq;
+  // Whether a box starting at t0, pushed now, would be the next one taken.
+  __device__ bool comes_first(float t0) const { return n == 0 || t0 <= e[n - 1].t0; }
+  __device__ IBox pop() { return e[--n]; }
+};
+
+// One search per warp, in the block's shared memory: a binary heap of 64-bit
+// keys (bits of t.lower >= 0, push sequence descending, slot of the box), so
+// a level of a pop moves one key, and the two children of a node are one
+// aligned load.  Lane 0 keeps it; every lane gets what is taken.
+struct WarpHeap {
+  static constexpr bool kWarp = true;
+  unsigned long long* key;  // 1-based, a key past the last is all ones
+  IBox* box;
+  int cap, n = 0, seq = 0, unused = 0, released = -1;
+  __device__ WarpHeap(unsigned char* mem, int capacity)
+      : key(reinterpret_cast<unsigned long long*>(mem)),
+        box(reinterpret_cast<IBox*>(mem + key_bytes(capacity))),
+        cap(capacity) {}
+  __host__ __device__ static size_t key_bytes(int capacity) {
+    return ((size_t)capacity + 3) / 2 * 16;
+  }
+  __host__ __device__ static size_t bytes(int capacity) {
+    return key_bytes(capacity) + (size_t)capacity * sizeof(IBox);
+  }
+  __device__ static bool lead() { return (threadIdx.x & 31) == 0; }
+  __device__ void reset() {
+    n = seq = unused = 0;
+    released = -1;
+  }
+  __device__ bool empty() const { return n == 0; }
+  __device__ bool push(const IBox& b) {
+    if (n >= cap) return false;
+    if (lead()) {
+      int slot = released;
+      if (slot >= 0)
+        released = __float_as_int(box[slot].t0);
+      else
+        slot = unused++;
+      box[slot] = b;
+      const unsigned long long k = (unsigned long long)__float_as_uint(b.t0) << 32 |
+                                   (unsigned)(0xffff - seq) << 16 | (unsigned)slot;
+      int i = n + 1;
+      key[i + 1] = ~0ull;
+      for (; i > 1 && k < key[i >> 1]; i >>= 1) key[i] = key[i >> 1];
+      key[i] = k;
     }
-    return top;
+    ++n;
+    ++seq;
+    return true;
+  }
+  __device__ bool comes_first(float t0) const {
+    int first = 0;
+    if (lead()) first = n == 0 || t0 <= __uint_as_float((unsigned)(key[1] >> 32));
+    return __shfl_sync(0xffffffffu, first, 0) != 0;
+  }
+  __device__ IBox pop() {
+    IBox b;
+    if (lead()) {
+      const int slot = (int)(key[1] & 0xffffu);
+      b = box[slot];
+      box[slot].t0 = __int_as_float(released);
+      released = slot;
+      const unsigned long long last = key[n];
+      key[n] = ~0ull;
+      if (n > 1) {
+        int i = 1;
+        while (2 * i < n) {
+          const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(key + 2 * i);
+          const unsigned long long k = c.x < c.y ? c.x : c.y;
+          if (last < k) break;
+          key[i] = k;
+          i = 2 * i + (c.x < c.y ? 0 : 1);
+        }
+        key[i] = last;
+      }
+    }
+    --n;
+    b.t0 = __shfl_sync(0xffffffffu, b.t0, 0);
+    b.t1 = __shfl_sync(0xffffffffu, b.t1, 0);
+    b.u0 = __shfl_sync(0xffffffffu, b.u0, 0);
+    b.u1 = __shfl_sync(0xffffffffu, b.u1, 0);
+    b.v0 = __shfl_sync(0xffffffffu, b.v0, 0);
+    b.v1 = __shfl_sync(0xffffffffu, b.v1, 0);
+    return b;
   }
 };
 
@@ -765,9 +805,14 @@ struct DfsStack {
 // t.lower > 0 with t.lower >= the smallest time of impact already found by
 // any query, no answer of this search can lower that minimum.  Stopping
 // there leaves the minimum over all queries bit-identical to the full search.
+//
+// With a warp's store every lane runs the search alike, lane d evaluates
+// dimension d (mod 3) and the lanes vote: the three dimensions of a box, one
+// after the other in a single thread, cost one evaluation.
+template <class Store>
 __device__ int root_finder(bool vf, const float3* Pt, const float* tol,
                            float co_tol, const float* err, float ms, int max_iter,
-                           float max_time, IBox& result, DfsStack& st,
+                           float max_time, IBox& result, Store& st,
                            const unsigned* best_bits = nullptr) {
   CcdCoeff co;
   for (int d = 0; d < 3; ++d) {
@@ -791,35 +836,52 @@ __device__ int root_finder(bool vf, const float3* Pt, const float* tol,
   bool unit = max_time == 1.0f;
   IBox cur{0.0f, max_time, 0.0f, 1.0f, 0.0f, 1.0f};
   bool has_cur = true;
-  st.n = 0;
-  st.seq = 0;
+  st.reset();
   int iter = 0;
+  const int my = (threadIdx.x & 31) % 3;  // dimension of this lane (warp store)
+  auto mine = [&](const float (&c)[3]) { return my == 0 ? c[0] : (my == 1 ? c[1] : c[2]); };
+  const float m0 = mine(co.c0), m1 = mine(co.c1), m2 = mine(co.c2), m3 = mine(co.c3),
+              m4 = mine(co.c4), m5 = mine(co.c5);
+  const float merr = my == 0 ? err[0] : (my == 1 ? err[1] : err[2]);
   auto push = [&](const IBox& b) -> bool { return st.push(b); };
   float best = __int_as_float(0x7f800000);
-  while (has_cur || st.n > 0) {
+  while (has_cur || !st.empty()) {
     if (!has_cur) cur = st.pop();
     has_cur = false;
     if (best_bits) {
-      if ((iter & 15) == 0) best = __uint_as_float(*(volatile const unsigned*)best_bits);
+      if ((iter & 15) == 0) {
+        best = __uint_as_float(*(volatile const unsigned*)best_bits);
+        if (Store::kWarp) best = __shfl_sync(0xffffffffu, best, 0);
+      }
       if (cur.t0 > 0.0f && cur.t0 >= best) return 3;
     }
     ++iter;
-    bool in_eps_all = true;
-    float w_img[3];
-    bool in_zero = true;
-    for (int d = 0; d < 3; ++d) {
-      bool ie;
-      bool ok = unit ? eval_unit_1d(vf, Pt, err[d], ms, d, ie, w_img[d])
-                     : eval_box_1d(vf, cur, co, err[d] + ms, d, ie, w_img[d]);
-      if (!ok) {
-        in_zero = false;
-        break;
+    bool in_eps_all = true, small = true, in_zero = true;
+    if (Store::kWarp) {
+      bool ie = false;
+      float w = 0.0f;
+      const bool ok = unit ? eval_unit_1d(vf, Pt, merr, ms, my, ie, w)
+                           : eval_box_1d(vf, cur, m0, m1, m2, m3, m4, m5, merr + ms, ie, w);
+      in_zero = __all_sync(0xffffffffu, ok);
+      in_eps_all = __all_sync(0xffffffffu, ie);
+      small = __all_sync(0xffffffffu, w <= co_tol);
+    } else {
+      for (int d = 0; d < 3; ++d) {
+        bool ie;
+        float w;
+        const bool ok = unit ? eval_unit_1d(vf, Pt, err[d], ms, d, ie, w)
+                             : eval_box_1d(vf, cur, co.c0[d], co.c1[d], co.c2[d], co.c3[d],
+                                           co.c4[d], co.c5[d], err[d] + ms, ie, w);
+        if (!ok) {
+          in_zero = false;
+          break;
+        }
+        in_eps_all = in_eps_all && ie;
+        small = small && w <= co_tol;
       }
-      in_eps_all = in_eps_all && ie;
     }
     unit = false;
     if (!in_zero) continue;
-    bool small = w_img[0] <= co_tol && w_img[1] <= co_tol && w_img[2] <= co_tol;
     if (small || in_eps_all) {
       result = cur;
       return 1;
@@ -859,7 +921,7 @@ __device__ int root_finder(bool vf, const float3* Pt, const float* tol,
     // pending store and straight back, which leaves the order of the search
     // unchanged.
     auto push_first = [&]() -> bool {
-      if (st.n == 0 || first.t0 <= st.top_t0()) {
+      if (st.comes_first(first.t0)) {
         cur = first;
         has_cur = true;
         return true;
@@ -887,9 +949,10 @@ __device__ int root_finder(bool vf, const float3* Pt, const float* tol,
 // Full query: tolerances, search, and the no-zero-toi refinement with half
 // the minimum separation (ccd.cpp:128-182).  Returns the status of the first
 // search; toi follows narrowphase.cu's use of the answer.
+template <class Store>
 __device__ int ccd_query(bool vf, const float3* Pt, const float* err, float ms,
                          float tolerance, int max_iter, float max_time, float& toi,
-                         float& t_upper, DfsStack& st,
+                         float& t_upper, Store& st,
                          const unsigned* best_bits = nullptr) {
   float3 p000, p001, p011, p010, p100, p101, p111, p110;
   if (vf) {
@@ -966,19 +1029,12 @@ struct CcdSpill {
   const int* list;    // second pass: query indices
   int* overflow;      // first pass: queries to re-run
   int* n_overflow;
-  int smem_heap = 0;  // second pass: one query per block, a heap of spill_cap
-                      // boxes in the block's shared memory (spill unused)
 };
 
 extern __shared__ __align__(16) unsigned char ccd_heap_smem[];
 
 __device__ __forceinline__ void bind_stack(DfsStack& st, const CcdSpill& sp, int i) {
-  if (sp.smem_heap) {
-    st.e = reinterpret_cast<IBox*>(ccd_heap_smem);
-    st.q = reinterpret_cast<int*>(ccd_heap_smem + (size_t)sp.spill_cap * sizeof(IBox));
-    st.cap = sp.spill_cap;
-    st.heap = true;
-  } else if (sp.spill) {
+  if (sp.spill) {
     st.e = sp.spill + (size_t)i * sp.spill_cap;
     st.cap = sp.spill_cap;
   } else {
@@ -987,11 +1043,11 @@ __device__ __forceinline__ void bind_stack(DfsStack& st, const CcdSpill& sp, int
   }
 }
 
-__device__ __noinline__ void ccd_one(const ObjDev* objs, const int4* cand, int i, float ts,
+template <class Store>
+__device__ __noinline__ void ccd_one(const ObjDev* objs, const int4* cand, int q, float ts,
                                      float interval, float ms, float3 vf_err, float3 ee_err,
                                      float local_tol, unsigned* min_bits, int* counts,
-                                     const CcdSpill& sp, int prune) {
-  int q = sp.list ? sp.list[i] : i;
+                                     const CcdSpill& sp, int prune, Store& st) {
   int4 c = cand[q];
   int kind = c.z >> 16, sa = c.z & 0xffff, sb = c.w;
   const ObjDev& A = objs[sa];
@@ -1016,14 +1072,13 @@ __device__ __noinline__ void ccd_one(const ObjDev* objs, const int4* cand, int i
   err[0] = e.x;
   err[1] = e.y;
   err[2] = e.z;
-  DfsStack st;
-  bind_stack(st, sp, i);
   float toi = 1.0f, tup = 1.0f;
   float local_max = interval / interval;
   int s = ccd_query(vf, Pt, err, ms, local_tol, kCcdMaxIter, local_max, toi, tup, st,
                     prune ? min_bits : nullptr);
+  if (Store::kWarp && (threadIdx.x & 31) != 0) return;
   if (s == 2) {
-    if (!sp.spill) sp.overflow[atomicAdd(sp.n_overflow, 1)] = q;
+    if (sp.overflow) sp.overflow[atomicAdd(sp.n_overflow, 1)] = q;
     else atomicAdd(&counts[1], 1);
     return;
   }
@@ -1044,53 +1099,111 @@ __global__ void __launch_bounds__(kCollThreads) ccd_kernel(
   for (;;) {
     int i = atomicAdd(next, 1);
     if (i >= n) return;
+    DfsStack st;
+    bind_stack(st, sp, i);
     ccd_one(objs, cand, i, ts, interval, ms, vf_err, ee_err, local_tol, min_bits, counts,
-            sp, prune);
+            sp, prune, st);
   }
 }
 
-// Second pass of the searches that outgrew the per-thread storage: one
-// query per block (block q takes list entry q), searched by thread 0 with
-// its pending boxes in a heap in the block's shared memory.
+// Second pass of the searches that outgrew the per-thread storage: one query
+// per warp and block (block i takes list entry i), its pending boxes in a
+// heap in the block's shared memory.  Bound by the latency of one evaluation
+// after the other, up to 4,096 and as many again for the refinement.  With
+// the search in one thread and whole boxes in the heap's nodes, the second
+// passes took 22 ms of a 41 x 41 sheet's first contact step, 14 ms now.  The
+// allocation-free batch kept 64 searches in sorted arrays in global memory:
+// 636 ms for 12,007 edge-edge queries with 60 deep ones, 8.6 ms here.
 __global__ void __launch_bounds__(32) ccd_heap_kernel(
     const ObjDev* objs, const int4* cand, int n, float ts, float interval, float ms,
     float3 vf_err, float3 ee_err, float local_tol, unsigned* min_bits, int* counts,
     CcdSpill sp, int prune) {
-  if (threadIdx.x != 0 || (int)blockIdx.x >= n) return;
-  ccd_one(objs, cand, blockIdx.x, ts, interval, ms, vf_err, ee_err, local_tol, min_bits, counts,
-          sp, prune);
+  if ((int)blockIdx.x >= n) return;
+  WarpHeap st(ccd_heap_smem, sp.spill_cap);
+  ccd_one(objs, cand, sp.list[blockIdx.x], ts, interval, ms, vf_err, ee_err, local_tol, min_bits,
+          counts, sp, prune, st);
 }
 
-constexpr size_t kCcdHeapSmemMax = 200 * 1024;  // heap second pass: up to ~7,300 boxes
+constexpr size_t kCcdHeapSmemMax = 226 * 1024;  // heap second pass: up to ~7,200 boxes
 
-size_t ccd_heap_smem_bytes(int cap) {
-  return (size_t)cap * (sizeof(IBox) + sizeof(int));
+template <class Store>
+__device__ int ccd_batch_query(bool vf, const float* x, int q, float3 err, const float* ms,
+                               float tol, int max_iter, float max_time, int* hit, float* toi,
+                               float* tup, Store& st) {
+  float3 Pt[8];
+  for (int k = 0; k < 8; ++k)
+    Pt[k] = make_float3(x[24 * q + 3 * k], x[24 * q + 3 * k + 1], x[24 * q + 3 * k + 2]);
+  float e[3] = {err.x, err.y, err.z};
+  float t = max_time, u = max_time;
+  int s = ccd_query(vf, Pt, e, ms[q], tol, max_iter, max_time, t, u, st);
+  if (s == 2 || (Store::kWarp && (threadIdx.x & 31) != 0)) return s;
+  hit[q] = s != 0 ? 1 : 0;
+  toi[q] = s != 0 ? t : max_time;
+  if (tup) tup[q] = s != 0 ? u : max_time;
+  return s;
 }
 
 __global__ void ccd_batch_kernel(bool vf, const float* x, int n, float3 err,
                                  const float* ms, float tol, int max_iter,
                                  float max_time, int* hit, float* toi, float* tup,
                                  int* n_bad, CcdSpill sp) {
-  int i = sp.smem_heap ? (threadIdx.x == 0 ? (int)blockIdx.x : n)
-                       : blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int q = sp.list ? sp.list[i] : i;
-  float3 Pt[8];
-  for (int k = 0; k < 8; ++k)
-    Pt[k] = make_float3(x[24 * q + 3 * k], x[24 * q + 3 * k + 1], x[24 * q + 3 * k + 2]);
-  float e[3] = {err.x, err.y, err.z};
   DfsStack st;
   bind_stack(st, sp, i);
-  float t = max_time, u = max_time;
-  int s = ccd_query(vf, Pt, e, ms[q], tol, max_iter, max_time, t, u, st);
-  if (s == 2) {
+  if (ccd_batch_query(vf, x, q, err, ms, tol, max_iter, max_time, hit, toi, tup, st) == 2) {
     if (!sp.spill) sp.overflow[atomicAdd(sp.n_overflow, 1)] = q;
     else atomicAdd(n_bad, 1);
-    return;
   }
-  hit[q] = s != 0 ? 1 : 0;
-  toi[q] = s != 0 ? t : max_time;
-  if (tup) tup[q] = s != 0 ? u : max_time;
+}
+
+// Second pass of a batch: blocks of one warp take the listed queries
+// (counters[0] of them) from a shared counter (counters[2]) and search them in
+// their shared memory.  A search that still runs out of storage (counters[1])
+// is answered with a hit at time 0, the conservative answer.
+__global__ void __launch_bounds__(32) ccd_batch_heap_kernel(
+    bool vf, const float* x, float3 err, const float* ms, float tol, int max_iter,
+    float max_time, int* hit, float* toi, float* tup, int* counters, const int* list, int cap) {
+  WarpHeap st(ccd_heap_smem, cap);
+  const int n = counters[0];
+  for (;;) {
+    int j = 0;
+    if (threadIdx.x == 0) j = atomicAdd(counters + 2, 1);
+    j = __shfl_sync(0xffffffffu, j, 0);
+    if (j >= n) return;
+    const int q = list[j];
+    const int s =
+        ccd_batch_query(vf, x, q, err, ms, tol, max_iter, max_time, hit, toi, tup, st);
+    if (s == 2 && threadIdx.x == 0) {
+      atomicAdd(counters + 1, 1);
+      hit[q] = 1;
+      toi[q] = 0.0f;
+      if (tup) tup[q] = max_time;
+    }
+    __syncwarp();
+  }
+}
+
+// Blocks of the batch's second pass: as many as are resident (one search a
+// block; its shared memory sets how many share an SM), or 0 when the storage
+// of a search does not fit one block.
+int ccd_batch_heap_blocks(int cap) {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    CUDA_CHECK(cudaGetDevice(&dev));
+    CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    CUDA_CHECK(cudaFuncSetAttribute(ccd_batch_heap_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kCcdHeapSmemMax));
+    return n;
+  }();
+  const size_t smem = WarpHeap::bytes(cap);
+  if (smem > kCcdHeapSmemMax) return 0;
+  int per_sm = 0;
+  CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ccd_batch_heap_kernel, 32,
+                                                           smem));
+  return sms * std::max(per_sm, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -2527,14 +2640,14 @@ float CollisionSystem::min_toi(float ts, float max_time, float ms, int* nq, int*
   // query per block, its pending boxes in a heap in shared memory.
   if (counts[2] > 0) {
     const int cap = kCcdMaxIter + 2;
-    const size_t smem = ccd_heap_smem_bytes(cap);
+    const size_t smem = WarpHeap::bytes(cap);
     static const bool attr = [smem] {
       CUDA_CHECK(cudaFuncSetAttribute(ccd_heap_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       return true;
     }();
     (void)attr;
-    CcdSpill second{nullptr, cap, I.ccd_overflow.p, nullptr, nullptr, 1};
+    CcdSpill second{nullptr, cap, I.ccd_overflow.p, nullptr, nullptr};
     ccd_heap_kernel<<<counts[2], 32, smem, st>>>(I.table_d.p, I.cand.p, counts[2], ts, max_time,
                                                  ms, vf, ee, local_tol, I.min_bits.p,
                                                  I.ccd_counts.p, second, prune ? 1 : 0);
@@ -2641,8 +2754,8 @@ void ccd_batch_host(bool vf, const float* x, int64_t n, const float* err3,
   CUDA_CHECK(cudaMemcpy(msd.p, ms, n * sizeof(float), cudaMemcpyHostToDevice));
   DevBuf<int> over, counts;
   over.alloc(n);
-  counts.alloc(2);
-  CUDA_CHECK(cudaMemset(counts.p, 0, 2 * sizeof(int)));
+  counts.alloc(3);
+  CUDA_CHECK(cudaMemset(counts.p, 0, 3 * sizeof(int)));
   float3 e3 = make_float3(err3[0], err3[1], err3[2]);
   CcdSpill first{nullptr, 0, nullptr, over.p, counts.p};
   ccd_batch_kernel<<<div_up((int)n, kCollThreads), kCollThreads>>>(
@@ -2656,20 +2769,11 @@ void ccd_batch_host(bool vf, const float* x, int64_t n, const float* err3,
     // Second pass with max_iter + 2 pending boxes per search (unbounded
     // searches, max_iter <= 0, get 65536).
     int cap = max_iter > 0 ? max_iter + 2 : 65536;
-    const size_t heap_smem = ccd_heap_smem_bytes(cap);
-    if (heap_smem <= kCcdHeapSmemMax) {
-      // One query per block, its pending boxes in a heap in shared memory.
-      static const bool attr = [] {
-        CUDA_CHECK(cudaFuncSetAttribute(ccd_batch_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kCcdHeapSmemMax));
-        return true;
-      }();
-      (void)attr;
-      CcdSpill second{nullptr, cap, over.p, nullptr, nullptr, 1};
-      ccd_batch_kernel<<<h[0], 32, heap_smem>>>(vf, xd.p, h[0], e3, msd.p, tol, max_iter,
-                                                max_time, hitd.p, toid.p, tupd.p, counts.p + 1,
-                                                second);
+    const int blocks = cap < 65536 ? ccd_batch_heap_blocks(cap) : 0;
+    if (blocks > 0) {
+      ccd_batch_heap_kernel<<<std::min(h[0], blocks), 32, WarpHeap::bytes(cap)>>>(
+          vf, xd.p, e3, msd.p, tol, max_iter, max_time, hitd.p, toid.p, tupd.p, counts.p, over.p,
+          cap);
       SILK_LAUNCHED();
     } else {
       int chunk =
@@ -2819,54 +2923,16 @@ int color_contacts_host(const int* verts4, const uint64_t* prio, int64_t n, int*
 //   [256, 256 + 4 MiB)       indices of the overflowed queries (written by
 //                            the first pass before they are read; no
 //                            initial value needed)
-//   [.., + 6,294,528 B)      pending-box storage of the second pass:
-//                            kNoAllocSpillSlots regions of max_iter + 2 boxes
-//                            (the most a search of max_iter steps can hold)
-// The first pass is ccd_batch_kernel itself; the second pass runs the
-// overflowed queries on kNoAllocSpillSlots threads that each reuse one
-// storage region, so the scratch size does not grow with the batch.
+// The first pass is ccd_batch_kernel itself; the second pass
+// (ccd_batch_heap_kernel) keeps its searches in shared memory, so the scratch
+// size does not grow with the batch.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr size_t kNoAllocListOffset = 256;
-constexpr size_t kNoAllocSpillOffset =
-    kNoAllocListOffset + sizeof(int) * (size_t)kNoAllocMaxQueries;
 constexpr size_t kNoAllocScratchBytes =
-    kNoAllocSpillOffset + sizeof(IBox) * (size_t)kNoAllocSpillSlots * (kNoAllocMaxIter + 2);
-static_assert(kNoAllocSpillOffset % 256 == 0, "spill region alignment");
+    kNoAllocListOffset + sizeof(int) * (size_t)kNoAllocMaxQueries;
 
 static __device__ __align__(256) unsigned char g_ccd_noalloc_scratch[kNoAllocScratchBytes];
-
-__global__ void __launch_bounds__(kNoAllocSpillSlots) ccd_batch_spill_kernel(
-    bool vf, const float* x, float3 err, const float* ms, float tol, int max_iter,
-    float max_time, int* hit, float* toi, float* tup, int* counters, const int* list,
-    IBox* spill) {
-  const int n_over = counters[0];
-  DfsStack st;
-  st.cap = max_iter + 2;
-  st.e = spill + (size_t)threadIdx.x * st.cap;
-  const float e[3] = {err.x, err.y, err.z};
-  for (;;) {
-    int j = atomicAdd(&counters[2], 1);
-    if (j >= n_over) return;
-    int q = list[j];
-    float3 Pt[8];
-    for (int k = 0; k < 8; ++k)
-      Pt[k] = make_float3(x[24 * q + 3 * k], x[24 * q + 3 * k + 1], x[24 * q + 3 * k + 2]);
-    float t = max_time, u = max_time;
-    int s = ccd_query(vf, Pt, e, ms[q], tol, max_iter, max_time, t, u, st);
-    if (s == 2) {
-      // Storage ran out: report the conservative answer (a hit at time 0).
-      atomicAdd(&counters[1], 1);
-      hit[q] = 1;
-      toi[q] = 0.0f;
-      if (tup) tup[q] = max_time;
-      continue;
-    }
-    hit[q] = s != 0 ? 1 : 0;
-    toi[q] = s != 0 ? t : max_time;
-    if (tup) tup[q] = s != 0 ? u : max_time;
-  }
-}
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mutex[kNoAllocMaxDevices];
@@ -2925,7 +2991,6 @@ NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float*
   unsigned char* base = g_noalloc_addr[dev];
   int* counters = reinterpret_cast<int*>(base);
   int* list = reinterpret_cast<int*>(base + kNoAllocListOffset);
-  IBox* spill = reinterpret_cast<IBox*>(base + kNoAllocSpillOffset);
   const float3 e3 = make_float3(err3[0], err3[1], err3[2]);
   // Any failure after work was queued waits for that work before returning,
   // so the lock is released only once the scratch array is idle.
@@ -2935,6 +3000,15 @@ NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float*
     cudaGetLastError();
     return NoAllocStatus::kCudaError;
   };
+  int heap_blocks = 0;
+  try {
+    heap_blocks = ccd_batch_heap_blocks(max_iter + 2);
+  } catch (const CudaError&) {
+  }
+  if (heap_blocks == 0) {
+    cudaGetLastError();
+    return NoAllocStatus::kCudaError;
+  }
   cudaGetLastError();  // an earlier, unrelated error is not this call's
   if (cudaMemsetAsync(counters, 0, 4 * sizeof(int), stream) != cudaSuccess)
     return fail_after_queue();
@@ -2943,8 +3017,8 @@ NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float*
       vf, x, (int)n, e3, ms, tol, max_iter, max_time, hit, toi, t_upper, counters + 1, first);
   SILK_LAUNCHED();
   if (cudaGetLastError() != cudaSuccess) return fail_after_queue();
-  ccd_batch_spill_kernel<<<1, kNoAllocSpillSlots, 0, stream>>>(
-      vf, x, e3, ms, tol, max_iter, max_time, hit, toi, t_upper, counters, list, spill);
+  ccd_batch_heap_kernel<<<heap_blocks, 32, WarpHeap::bytes(max_iter + 2), stream>>>(
+      vf, x, e3, ms, tol, max_iter, max_time, hit, toi, t_upper, counters, list, max_iter + 2);
   SILK_LAUNCHED();
   if (cudaGetLastError() != cudaSuccess) return fail_after_queue();
   int h[4] = {0, 0, 0, 0};

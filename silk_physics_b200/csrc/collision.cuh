@@ -86,7 +86,6 @@ void coulomb_debug_host(const float* u, const float* nrm, const float* mu, int64
 // allocates no memory: all working memory is a static device array.
 constexpr int kNoAllocMaxQueries = 1 << 20;
 constexpr int kNoAllocMaxIter = 4096;
-constexpr int kNoAllocSpillSlots = 64;
 enum class NoAllocStatus { kOk, kBadArgument, kBeyondLimits, kCudaError, kStorageExhausted };
 NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float* err3,
                                 const float* ms, float tol, int max_iter, float max_time,

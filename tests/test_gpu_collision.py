@@ -4,6 +4,7 @@ valid and identical; full steps with contacts stay within tolerance."""
 import numpy as np
 import pytest
 
+import ccd_cases as CC
 from silk_physics_b200 import native as N
 from silk_physics_b200 import scenes as S
 
@@ -334,3 +335,39 @@ def test_gs_single_block_sizes_identical(s, so, few, many):
     assert few <= out[0][1] <= many
     assert out[0][1] == out[1][1]
     np.testing.assert_array_equal(out[0][0], out[1][0])
+
+
+# Pending-box stores of the deep searches: 96 per thread in the first pass,
+# heaps in shared memory (up to about 7,200 boxes), sorted arrays in global
+# memory above that; the smallest cap, around the first pass's size, and both
+# sides of the shared-memory limit.
+@pytest.mark.parametrize("max_iter", [1, 94, 95, 96, 300, 7000, 7400])
+@pytest.mark.parametrize("vf", [True, False])
+def test_ccd_deep_search_stores_match_oracle(oracle, vf, max_iter):
+    """Near-contact queries (searches of up to max_iter evaluations): hit,
+    time of impact and upper bound equal the CPU restatement's bit for bit,
+    whichever store holds the pending boxes; the allocation-free batch gives
+    the same answers within its limit of 4,096."""
+    import torch
+    rng = np.random.default_rng(77)
+    x = CC.near_contact_queries(rng, 40, vf)
+    ms = np.full(40, 1e-3, np.float32)
+    err = [CC.ERR[vf]] * 3
+    hit, toi, tup = N.ccd_batch(vf, x, err, ms, max_iter=max_iter)
+    for i in range(40):
+        h, t = oracle.ccd_toi(vf, x[i], err, float(ms[i]), max_iter=max_iter)[:2]
+        assert bool(h) == bool(hit[i])
+        if h:
+            assert np.float32(t) == toi[i]
+    if max_iter > 4096:
+        return
+    d = {k: torch.from_numpy(v).cuda() for k, v in (("x", x), ("ms", ms))}
+    o = [torch.zeros(40, dtype=t, device="cuda") for t in (torch.int32, torch.float32,
+                                                           torch.float32)]
+    r, _ = N.ccd_batch_noalloc(vf, d["x"].data_ptr(), 40, np.asarray(err, np.float32),
+                               d["ms"].data_ptr(), *(b.data_ptr() for b in o),
+                               max_iter=max_iter)
+    assert r, r.to_string()
+    np.testing.assert_array_equal(o[0].cpu().numpy().astype(bool), hit)
+    np.testing.assert_array_equal(o[1].cpu().numpy(), toi)
+    np.testing.assert_array_equal(o[2].cpu().numpy(), tup)
