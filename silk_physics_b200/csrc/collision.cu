@@ -1289,64 +1289,80 @@ __global__ void activate_weights_kernel(const int* count, int nv, const float* b
   if (threadIdx.x == 0 && act) atomicAdd(active_dof, 3 * act);
 }
 
-// One Jones-Plassmann round: a contact whose higher-priority neighbours are
-// all coloured takes the smallest colour none of them uses.
-// One Jones-Plassmann step of contact i: 0 when a higher-priority neighbour
-// (sharing a movable vertex) is still uncoloured, else the smallest colour
-// none of them holds (1025 past 1,024 colours).  A neighbour coloured in the
-// same round may or may not be seen; either way contact i ends with the
-// smallest colour its higher-priority neighbours leave free, so the result
-// is the sequential greedy colouring in priority order.
+// One Jones-Plassmann step of contact i by one warp: 0 when a higher-priority
+// neighbour (sharing a movable vertex) is still uncoloured, else the smallest
+// colour none of them holds (1025 past 1,024 colours).  A neighbour coloured
+// in the same round may or may not be seen; either way contact i ends with
+// the smallest colour its higher-priority neighbours leave free, so the
+// result is the sequential greedy colouring in priority order.  The lanes
+// share the neighbours (up to four vertices with a hundred contacts each) and
+// mark their colours in `used`, 32 words of shared memory.
 __device__ int jp_pick(const ContactDev* c, const unsigned long long* prio, int i,
-                       const int* off, const int* list, const int* color) {
-  unsigned long long pi = prio[i];
-  unsigned used[32];
-  for (int k = 0; k < 32; ++k) used[k] = 0u;
+                       const int* off, const int* list, const int* color, unsigned* used) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long pi = prio[i];
+  used[lane] = 0u;
+  __syncwarp();
+  bool wait = false;
   for (int s = 0; s < 4; ++s) {
     if (c[i].gamma[s] == 0.0f) continue;
-    int v = c[i].v[s];
-    for (int q = off[v]; q < off[v + 1]; ++q) {
-      int j = list[q];
+    const int v = c[i].v[s];
+    for (int q = off[v] + lane; q < off[v + 1]; q += 32) {
+      const int j = list[q];
       if (j == i) continue;
-      unsigned long long pj = prio[j];
-      bool higher = pj > pi || (pj == pi && j < i);
-      if (!higher) continue;
-      int cj = ((const volatile int*)color)[j];
-      if (cj == 0) return 0;
-      if (cj <= 1024) used[(cj - 1) >> 5] |= 1u << ((cj - 1) & 31);
+      const unsigned long long pj = prio[j];
+      if (!(pj > pi || (pj == pi && j < i))) continue;
+      const int cj = ((const volatile int*)color)[j];
+      if (cj == 0)
+        wait = true;
+      else if (cj <= 1024)
+        atomicOr(used + ((cj - 1) >> 5), 1u << ((cj - 1) & 31));
     }
   }
-  int col = 0;
-  for (int k = 0; k < 32 && col == 0; ++k)
-    if (used[k] != 0xffffffffu) col = 32 * k + __ffs(~used[k]);
-  return col == 0 ? 1025 : col;
+  const bool blocked = __any_sync(0xffffffffu, wait);
+  __syncwarp();
+  const unsigned mine = used[lane];
+  const unsigned open = __ballot_sync(0xffffffffu, mine != 0xffffffffu);
+  if (blocked) return 0;
+  if (open == 0u) return 1025;
+  const int word = __ffs(open) - 1;
+  return 32 * word + __ffs(~__shfl_sync(0xffffffffu, mine, word));
 }
 
-// Every round in one cooperative launch: one thread per contact (grid-
-// stride), the bounded grid barrier between rounds instead of launches and
-// host checks.  Round r counts its uncoloured contacts in rem[r % 3]; the
-// counter of round r + 1 is cleared during round r, after every block has
-// read it for round r - 2.  info: [0] highest colour, [1] contacts past
-// 1,024 colours, [3] set when a barrier wait gave up or the rounds ran out.
+// Every round in one cooperative launch: one warp per contact (grid-stride),
+// the bounded grid barrier between rounds instead of launches and host
+// checks.  Round r counts its uncoloured contacts in rem[r % 3]; the counter
+// of round r + 1 is cleared during round r, after every block has read it for
+// round r - 2.  info: [0] highest colour, [1] contacts past 1,024 colours,
+// [3] set when a barrier wait gave up or the rounds ran out.  Bound by the
+// rounds (the longest chain of ever higher priorities) times one scan of a
+// contact's neighbours; with a thread per contact that scan was serial (2.0 ms
+// a call for 519 contacts in 75 colours, 11 ms of that step more than now).
 constexpr int kJpMaxRounds = 4096;
-__global__ void jp_grid_kernel(const ContactDev* c, const unsigned long long* prio, int n,
-                               const int* off, const int* list, int* color, int* info, int* rem,
-                               unsigned* barrier, long long spin_limit) {
+constexpr int kJpThreads = 256;
+__global__ void __launch_bounds__(kJpThreads) jp_grid_kernel(
+    const ContactDev* c, const unsigned long long* prio, int n, const int* off, const int* list,
+    int* color, int* info, int* rem, unsigned* barrier, long long spin_limit) {
   GridBarrier bar{barrier, barrier + 1, barrier + 2, gridDim.x};
   if (spin_limit > 0) bar.limit = spin_limit;
-  const int stride = gridDim.x * blockDim.x;
+  __shared__ unsigned used[kJpThreads / 32][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int stride = gridDim.x * (kJpThreads / 32);
   for (int round = 0; round < kJpMaxRounds; ++round) {
     if (blockIdx.x == 0 && threadIdx.x == 0) rem[(round + 1) % 3] = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-      if (color[i] != 0) continue;
-      const int col = jp_pick(c, prio, i, off, list, color);
-      if (col == 0) {
-        atomicAdd(rem + round % 3, 1);
-        continue;
+    for (int i = blockIdx.x * (kJpThreads / 32) + warp; i < n; i += stride) {
+      if (((const volatile int*)color)[i] != 0) continue;  // set by this warp alone
+      const int col = jp_pick(c, prio, i, off, list, color, used[warp]);
+      if (lane == 0) {
+        if (col == 0) {
+          atomicAdd(rem + round % 3, 1);
+        } else {
+          if (col > 1024) atomicAdd(info + 1, 1);
+          atomicMax(info, col);
+          ((volatile int*)color)[i] = col;
+        }
       }
-      if (col > 1024) atomicAdd(info + 1, 1);
-      atomicMax(info, col);
-      color[i] = col;
+      __syncwarp();
     }
     if (!bar.sync()) {
       if (blockIdx.x == 0 && threadIdx.x == 0) info[3] = 1;  // a barrier wait gave up
@@ -2417,10 +2433,12 @@ int CollisionSystem::append_active(float time, float dact) {
       int dev = 0, sms = 0, per = 0;
       CUDA_CHECK(cudaGetDevice(&dev));
       CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, jp_grid_kernel, 256, 0));
-      return sms * std::max(per, 1);
+      CUDA_CHECK(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, jp_grid_kernel, kJpThreads, 0));
+      return sms * std::min(std::max(per, 1), 2);
     }();
-    const int grid = std::min(max_coop, std::max(1, div_up(total, 256)));
+    // A warp per contact up to two blocks an SM (more only slow the barrier).
+    const int grid = std::min(max_coop, std::max(1, div_up(total, kJpThreads / 32)));
     CUDA_CHECK(cudaMemsetAsync(I.jp_flags.p, 0, 3 * sizeof(int), st));
     CUDA_CHECK(cudaMemsetAsync(I.gs_barrier.p, 0, 2 * sizeof(unsigned), st));
     const ContactDev* cp = I.contacts.p;
@@ -2434,7 +2452,7 @@ int CollisionSystem::append_active(float time, float dact) {
     unsigned* barp = I.gs_barrier.p;
     long long limit = w_.opt.barrier_spin_limit;
     void* args[] = {&cp, &pp, &n, &op, &lp, &colp, &infop, &remp, &barp, &limit};
-    CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)jp_grid_kernel, dim3(grid), dim3(256),
+    CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)jp_grid_kernel, dim3(grid), dim3(kJpThreads),
                                            args, 0, st));
     SILK_LAUNCHED();
   }
