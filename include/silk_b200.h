@@ -90,7 +90,10 @@ typedef struct {
   int32_t cg_form;            /* 0: the cluster form with redundant coarse
                                  levels where the system fits one cluster of
                                  CTAs of 8 or 16 fine banks, else the resident
-                                 form where it fits, else streaming;
+                                 form where it fits, else streaming, and from
+                                 the 16th iteration of an ADMM solve on the
+                                 direct form in place of the CG (the other
+                                 values never use it);
                                  2: resident where it fits, else streaming;
                                  1: streaming always;
                                  3, 4: as 0 and 2, the cluster and resident
@@ -146,8 +149,9 @@ typedef struct {
   int64_t cg_launches;
   int64_t cg_iterations;
   double cg_algorithmic_bytes;
-  double admm_other_ms;      /* events: face/vertex/contact kernels and the
-                                convergence test run by the vertex step */
+  double admm_other_ms;      /* events: face/vertex/contact kernels, the
+                                convergence test run by the vertex step and
+                                the direct solves */
   double admm_host_ms;       /* host wall time of ADMM control (syncs) */
   double ccd_host_ms;        /* host wall time of refit + CCD */
   double dcd_host_ms;        /* host wall time of DCD + contact rebuild */
@@ -172,8 +176,10 @@ typedef struct {
 typedef struct {
   int32_t outer_iterations;
   int32_t admm_iterations;
-  int32_t cg_iterations;
-  int32_t cg_solves;
+  int32_t cg_iterations;       /* of the systems that the CG solved */
+  int32_t cg_solves;           /* systems solved by CG; those of a long ADMM
+                                  solve's later iterations are solved directly
+                                  (cg_form 0) and counted in neither */
   int32_t contacts;
   int32_t colors;
   int32_t ccd_queries;
