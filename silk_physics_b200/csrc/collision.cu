@@ -35,6 +35,7 @@
 
 #include "collision.cuh"
 #include "grid_barrier.cuh"
+#include "per_device.hpp"
 #include "world.hpp"
 
 namespace silkb {
@@ -1185,25 +1186,26 @@ __global__ void __launch_bounds__(32) ccd_batch_heap_kernel(
   }
 }
 
-// Blocks of the batch's second pass: as many as are resident (one search a
-// block; its shared memory sets how many share an SM), or 0 when the storage
-// of a search does not fit one block.
+// Blocks of the batch's second pass: as many as are resident on the current
+// device (one search a block; its shared memory sets how many share an SM),
+// or 0 when the storage of a search does not fit one block.
 int ccd_batch_heap_blocks(int cap) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
-    CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  static PerDevice<int> sms;
+  const int dev = current_device();
+  const int n = sms.get(dev, [dev] {
+    int count = 0;
+    CUDA_CHECK(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
     CUDA_CHECK(cudaFuncSetAttribute(ccd_batch_heap_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kCcdHeapSmemMax));
-    return n;
-  }();
+    return count;
+  });
   const size_t smem = WarpHeap::bytes(cap);
   if (smem > kCcdHeapSmemMax) return 0;
   int per_sm = 0;
   CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ccd_batch_heap_kernel, 32,
                                                            smem));
-  return sms * std::max(per_sm, 1);
+  return n * per_sm;
 }
 
 // ---------------------------------------------------------------------------
@@ -2429,14 +2431,15 @@ int CollisionSystem::append_active(float time, float dact) {
   I.colors.zero(st);
   I.col_info.zero(st);
   {
-    static const int max_coop = [] {
-      int dev = 0, sms = 0, per = 0;
-      CUDA_CHECK(cudaGetDevice(&dev));
+    static PerDevice<int> coop;
+    const int dev = current_device();
+    const int max_coop = coop.get(dev, [dev] {
+      int sms = 0, per = 0;
       CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       CUDA_CHECK(
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, jp_grid_kernel, kJpThreads, 0));
       return sms * std::min(std::max(per, 1), 2);
-    }();
+    });
     // A warp per contact up to two blocks an SM (more only slow the barrier).
     const int grid = std::min(max_coop, std::max(1, div_up(total, kJpThreads / 32)));
     CUDA_CHECK(cudaMemsetAsync(I.jp_flags.p, 0, 3 * sizeof(int), st));
@@ -2552,13 +2555,13 @@ void CollisionSystem::contact_solve_launch() {
   const size_t pos = (size_t)(I.gs_nslots + 1) * sizeof(float4);
   const size_t both = pos + (size_t)I.n_contacts * sizeof(float4);
   if (I.gs_ready && w_.opt.contact_gs_form != 1 && pos <= kGsBlockSmemMax) {
-    static const bool attr = [] {
+    static PerDevice<bool> opted;
+    opted.get(current_device(), [] {
       for (auto* k : {contact_gs_flow_kernel<true>, contact_gs_flow_kernel<false>})
         CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kGsBlockSmemMax));
       return true;
-    }();
-    (void)attr;
+    });
     const bool shared = both <= kGsBlockSmemMax;
     // About six batches a warp: fewer leave warps polling beside the ones
     // that work, more put contacts that could run behind ones that wait
@@ -2574,13 +2577,14 @@ void CollisionSystem::contact_solve_launch() {
     SILK_LAUNCHED();
     return;
   }
-  static const int max_coop = [] {
-    int dev = 0, sms = 0, per = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+  static PerDevice<int> coop;
+  const int dev = current_device();
+  const int max_coop = coop.get(dev, [dev] {
+    int sms = 0, per = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, contact_gs_kernel, 256, 0));
     return sms * std::max(per, 1);
-  }();
+  });
   int grid = std::min(max_coop, std::max(1, div_up(I.max_group, 256)));
   CUDA_CHECK(cudaMemsetAsync(I.gs_barrier.p, 0, 2 * sizeof(unsigned), st));
   const ContactDev* c = I.contacts.p;
@@ -2632,12 +2636,13 @@ float CollisionSystem::min_toi(float ts, float max_time, float ms, int* nq, int*
   // counts: [hits, storage overflows, first-pass spills, work counter]
   CUDA_CHECK(cudaMemsetAsync(I.ccd_counts.p, 0, 4 * sizeof(int), st));
   if ((int)I.ccd_overflow.n < n) I.ccd_overflow.alloc(n + n / 4);
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+  static PerDevice<int> sm_count;
+  const int dev = current_device();
+  const int sms = sm_count.get(dev, [dev] {
+    int n = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     return n;
-  }();
+  });
   auto grid_for = [&](int m) { return std::max(1, std::min(div_up(m, kCollThreads), 8 * sms)); };
   if (!I.ccd_ev[0]) {
     for (auto& e : I.ccd_ev) CUDA_CHECK(cudaEventCreate(&e));
@@ -2659,12 +2664,12 @@ float CollisionSystem::min_toi(float ts, float max_time, float ms, int* nq, int*
   if (counts[2] > 0) {
     const int cap = kCcdMaxIter + 2;
     const size_t smem = WarpHeap::bytes(cap);
-    static const bool attr = [smem] {
+    static PerDevice<bool> opted;
+    opted.get(dev, [smem] {
       CUDA_CHECK(cudaFuncSetAttribute(ccd_heap_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       return true;
-    }();
-    (void)attr;
+    });
     CcdSpill second{nullptr, cap, I.ccd_overflow.p, nullptr, nullptr};
     ccd_heap_kernel<<<counts[2], 32, smem, st>>>(I.table_d.p, I.cand.p, counts[2], ts, max_time,
                                                  ms, vf, ee, local_tol, I.min_bits.p,
@@ -2793,6 +2798,7 @@ void ccd_batch_host(bool vf, const float* x, int64_t n, const float* err3,
           vf, xd.p, e3, msd.p, tol, max_iter, max_time, hitd.p, toid.p, tupd.p, counts.p, over.p,
           cap);
       SILK_LAUNCHED();
+      CUDA_CHECK(cudaGetLastError());
     } else {
       int chunk =
           std::max(1, std::min(h[0], (int)((256ll << 20) / ((long long)cap * sizeof(IBox)))));
@@ -2805,6 +2811,7 @@ void ccd_batch_host(bool vf, const float* x, int64_t n, const float* err3,
             vf, xd.p, m, e3, msd.p, tol, max_iter, max_time, hitd.p, toid.p, tupd.p,
             counts.p + 1, second);
         SILK_LAUNCHED();
+        CUDA_CHECK(cudaGetLastError());
       }
     }
     CUDA_CHECK(cudaMemcpy(h, counts.p, sizeof(h), cudaMemcpyDeviceToHost));
@@ -2966,6 +2973,15 @@ bool device_buffer(const void* p, int dev) {
   if (a.type == cudaMemoryTypeManaged) return true;
   return a.type == cudaMemoryTypeDevice && a.device == dev;
 }
+
+// Blocks of the second pass on the current device, 0 where it cannot run.
+int noalloc_heap_blocks(int max_iter) {
+  try {
+    return ccd_batch_heap_blocks(max_iter + 2);
+  } catch (const CudaError&) {
+    return 0;
+  }
+}
 }  // namespace
 
 NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float* err3,
@@ -2992,9 +3008,11 @@ NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float*
   std::lock_guard<std::mutex> lock(g_noalloc_mutex[dev]);
   if (!g_noalloc_addr[dev]) {
     // One-time setup on this device (the device is current): resolving the
-    // symbol loads this module's kernels and its scratch array.
+    // symbol loads this module's kernels and its scratch array, and the
+    // second pass opts in to its shared memory.
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_ccd_noalloc_scratch) != cudaSuccess || !p) {
+    if (cudaGetSymbolAddress(&p, g_ccd_noalloc_scratch) != cudaSuccess || !p ||
+        noalloc_heap_blocks(kNoAllocMaxIter) == 0) {
       cudaGetLastError();
       return NoAllocStatus::kCudaError;
     }
@@ -3018,11 +3036,7 @@ NoAllocStatus ccd_batch_noalloc(bool vf, const float* x, int64_t n, const float*
     cudaGetLastError();
     return NoAllocStatus::kCudaError;
   };
-  int heap_blocks = 0;
-  try {
-    heap_blocks = ccd_batch_heap_blocks(max_iter + 2);
-  } catch (const CudaError&) {
-  }
+  const int heap_blocks = noalloc_heap_blocks(max_iter);
   if (heap_blocks == 0) {
     cudaGetLastError();
     return NoAllocStatus::kCudaError;

@@ -23,6 +23,12 @@ inline void check_cuda(cudaError_t e, const char* what) {
 }
 #define CUDA_CHECK(x) ::silkb::check_cuda((x), #x)
 
+inline int current_device() {
+  int dev = 0;
+  CUDA_CHECK(cudaGetDevice(&dev));
+  return dev;
+}
+
 // Counts every kernel launch issued by this library (reported in the per-step
 // statistics so callers can see how many native kernels a step took).
 extern thread_local long long g_launch_count;

@@ -1,4 +1,7 @@
 """Host-side setup checked against the oracle (no GPU needed)."""
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -172,3 +175,15 @@ def test_resident_row_schedule():
     print(f"quarter passes: in row order {plain}, scheduled {sched}, minimum {ideal}")
     assert sched <= 1.1 * ideal
     assert plain >= 1.5 * ideal
+
+
+def test_values_belong_to_one_device(tmp_path):
+    """Kernel attributes and grid limits are kept per device: made once for
+    each, not once for the process."""
+    root = Path(__file__).resolve().parent
+    exe = tmp_path / "per_device"
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-pthread", "-I",
+                    str(root.parent / "silk_physics_b200" / "csrc"),
+                    str(root / "cpp" / "per_device.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and "ok" in out.stdout, out

@@ -100,3 +100,31 @@ def test_noalloc_refuses_sizes_beyond_limits():
     # n == 0 is a valid no-op.
     st, spilled = N.ccd_batch_noalloc(True, p, 0, err, p, ip, p, None)
     assert st and spilled == 0
+
+
+def test_noalloc_on_every_device():
+    """The second pass's shared-memory opt-in and the scratch address belong
+    to a device: after a call on device 0 the same queries give the same
+    answers on device 1."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one device")
+    rng = np.random.default_rng(142)
+    n = 3000
+    x = _queries(rng, n, True)
+    err = np.array([4.053116e-06] * 3, np.float32)
+    ms = rng.choice([0.0, 1e-4, 1e-3], n).astype(np.float32)
+    out = []
+    for k in range(2):
+        with torch.cuda.device(k):
+            d = [torch.from_numpy(a).cuda() for a in (x, ms)]
+            o = [torch.zeros(n, dtype=t, device="cuda") for t in (torch.int32, torch.float32,
+                                                                  torch.float32)]
+            st, spilled = N.ccd_batch_noalloc(True, d[0].data_ptr(), n, err, d[1].data_ptr(),
+                                              *(b.data_ptr() for b in o))
+            assert st, st.to_string()
+            out.append([spilled] + [b.cpu().numpy() for b in o])
+    assert out[0][0] > 0 and out[1][0] == out[0][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        np.testing.assert_array_equal(a, b)
