@@ -24,6 +24,7 @@
 #include "direct.cuh"
 #include "grid_barrier.cuh"
 #include "mas_cg.cuh"
+#include "per_device.hpp"
 
 namespace silkb {
 
@@ -590,14 +591,15 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
 }  // namespace
 
 int direct_max_blocks(size_t smem) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+  static PerDevice<int> sm_count;
+  const int dev = current_device();
+  const int sms = sm_count.get(dev, [dev] {
+    int n = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     CUDA_CHECK(cudaFuncSetAttribute(direct_solve_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return n;
-  }();
+  });
   int per_sm = 0;
   if (smem > 200 * 1024 ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, direct_solve_kernel, kDirectThreads,

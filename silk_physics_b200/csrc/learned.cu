@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 
 #include "learned.cuh"
+#include "per_device.hpp"
 
 namespace silkb {
 
@@ -670,12 +671,13 @@ __global__ void iterate_sample_kernel(int m, int n, unsigned salt, const float* 
 // most 4 per SM (256 threads, ~37 KB of shared memory and 64 tensor-memory
 // columns each).
 int tc_grid(int n) {
-  static const int max_grid = [] {
-    int dev = 0, sms = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+  static PerDevice<int> grid;
+  const int dev = current_device();
+  const int max_grid = grid.get(dev, [dev] {
+    int sms = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     return 4 * sms;
-  }();
+  });
   const int tiles = (n + kTcRows - 1) / kTcRows;
   return tiles < 1 ? 1 : (tiles < max_grid ? tiles : max_grid);
 }
@@ -712,13 +714,13 @@ void mlp_loss_grad(const MlpDev& m, const float* feat, const float* t_hat, int n
   mlp_forward_tc_kernel<true><<<fg, kTcThreads, sizeof(TcSmem), st>>>(
       m, feat, n, nullptr, m.fail, t_hat, index, z, d4, loss_part);
   SILK_LAUNCHED();
-  static const bool attr = [] {
+  static PerDevice<bool> opted;
+  opted.get(current_device(), [] {
     CUDA_CHECK(cudaFuncSetAttribute(mlp_backward_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(BwdSmem)));
     return true;
-  }();
-  (void)attr;
+  });
   mlp_backward_kernel<<<kBwdBlocks, kBwdThreads, sizeof(BwdSmem), st>>>(m, feat, index, n, z, d4,
                                                                         part);
   SILK_LAUNCHED();

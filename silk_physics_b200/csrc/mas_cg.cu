@@ -25,6 +25,7 @@
 
 #include "grid_barrier.cuh"
 #include "mas_cg.cuh"
+#include "per_device.hpp"
 
 namespace silkb {
 
@@ -1347,7 +1348,8 @@ __global__ void __launch_bounds__(kResThreads, 1) cg_resident_cluster_kernel(CgA
 }
 
 int max_cluster_size() {
-  static const int size = [] {
+  static PerDevice<int> size;
+  return size.get(current_device(), [] {
     size_t smem = kCgWarps * kPacked * sizeof(float);
     if (cudaFuncSetAttribute(cg_kernel_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed,
                              1) != cudaSuccess) {
@@ -1370,8 +1372,7 @@ int max_cluster_size() {
       n = 8;
     }
     return n >= 16 ? 16 : (n >= 8 ? 8 : 0);
-  }();
-  return size;
+  });
 }
 
 
@@ -1980,7 +1981,8 @@ size_t dsm_smem_bytes() {
 
 template <int F>
 int dsm_max_cluster() {
-  static const int n = [] {
+  static PerDevice<int> size;
+  return size.get(current_device(), [] {
     const size_t smem = sizeof(DsmShared<F>);
     if (cudaFuncSetAttribute(cg_dsm_cluster_kernel<F>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -2007,8 +2009,7 @@ int dsm_max_cluster() {
       m = 0;
     }
     return m < kDsmMaxCtas ? m : kDsmMaxCtas;
-  }();
-  return n;
+  });
 }
 
 template <int F>
@@ -2052,15 +2053,16 @@ int cg_grid_size(int nslices, int nbank0) {
   int cl = max_cluster_size();
   // One cluster while each warp has at most ~3 slices / banks to process.
   if (cl > 0 && want_blocks <= 3 * cl) return -cl;
-  static const int max_coop = [] {
-    int dev = 0, sms = 0, per_sm = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+  static PerDevice<int> coop;
+  const int dev = current_device();
+  const int max_coop = coop.get(dev, [dev] {
+    int sms = 0, per_sm = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     size_t smem = kCgWarps * kPacked * sizeof(float);
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_kernel,
                                                              kCgThreads, smem));
     return sms * (per_sm > 0 ? per_sm : 1);
-  }();
+  });
   int want = div_up(nslices > nbank0 ? nslices : nbank0, kCgWarps);
   if (want < 1) want = 1;
   return want < max_coop ? want : max_coop;
@@ -2096,11 +2098,12 @@ int cg_resident_grid(int res_blocks) {
   struct Limits {
     int max_coop = 0, max_cluster = 0;
   };
-  static const Limits lim = [] {
+  static PerDevice<Limits> limits;
+  const int dev = current_device();
+  const Limits lim = limits.get(dev, [dev] {
     Limits l;
     const size_t smem = sizeof(ResShared);
-    int dev = 0, sms = 0, per_sm = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
+    int sms = 0, per_sm = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CUDA_CHECK(cudaFuncSetAttribute(cg_resident_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2134,7 +2137,7 @@ int cg_resident_grid(int res_blocks) {
     }
     l.max_cluster = n >= 16 ? 16 : (n >= 8 ? 8 : 0);
     return l;
-  }();
+  });
   if (res_blocks <= 0 || lim.max_coop == 0) return 0;
   if (res_blocks > 1 && res_blocks <= lim.max_cluster) return -res_blocks;
   return res_blocks <= lim.max_coop ? res_blocks : 0;

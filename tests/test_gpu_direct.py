@@ -93,3 +93,30 @@ def test_direct_form_leaves_what_it_cannot_meet_to_the_cg():
         assert w.get_cloth_position(h, x)
         out.append(x)
     np.testing.assert_array_equal(out[0], out[1])
+
+
+def test_direct_form_on_every_device():
+    """Resident-block limits and shared-memory opt-ins belong to a device: the
+    same scene on device 1 is solved directly as on device 0, to the bit."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one device")
+    V, F = S.grid_sheet(60, jitter=1e-4, seed=3)
+    out = []
+    for dev in range(2):
+        with torch.cuda.device(dev):
+            w = N.World()
+            assert w.init()
+            assert w.set_global_config(N.GlobalConfig(max_inner_iteration=24, admm_abs_tol=0.0,
+                                                      admm_rel_tol=0.0))
+            assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5))
+            r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+                is_collision_on=False, is_self_collision_on=False), V, F, S.top_corner_pins(60))
+            assert r
+            assert w.solver_step()
+            assert w.step_stats().cg_solves == DIRECT_FROM - 1
+            x = np.zeros(V.size, np.float32)
+            assert w.get_cloth_position(h, x)
+            out.append(x)
+    np.testing.assert_array_equal(out[0], out[1])
