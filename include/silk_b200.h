@@ -124,12 +124,12 @@ typedef struct {
                                  through the grid (applies when the solver
                                  layout is built: first step after a change of
                                  the cloths); 0: 1024 */
-  int32_t barrier_spin_limit; /* > 0: polls after which a CG grid-barrier wait
-                                 gives up (the step then returns
+  int32_t barrier_spin_limit; /* > 0: polls after which a grid-barrier wait of
+                                 the CG or the direct form gives up (the step then returns
                                  SILK_ERR_ITERATIVE_SOLVE_FAIL); 0: 2^22 */
   int32_t debug_withhold_block; /* failure-detection tests: k > 0 makes block
-                                 k - 1 of a cooperative-grid CG launch skip its
-                                 barrier arrivals, so the other blocks' bounded
+                                 k - 1 of a cooperative-grid CG launch or direct
+                                 solve skip its barrier arrivals, so the other blocks' bounded
                                  waits run out; 0: off */
   int32_t admm_check_interval; /* ADMM iterations enqueued between the host's
                                  reads of the convergence state (the device

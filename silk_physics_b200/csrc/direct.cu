@@ -543,11 +543,14 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
   extern __shared__ float4 sm[];
   GridBarrier bar{a.barrier, a.barrier + 1, nullptr, gridDim.x};
   if (a.barrier_spin_limit > 0) bar.limit = a.barrier_spin_limit;
+  if (a.withhold_block >= 0) bar.withhold = (unsigned)a.withhold_block;
+  // Reported by every block whose wait gave up: block 0's own may have
+  // succeeded on the same barrier.
   auto sync = [&]() {
     if (bar.sync()) return true;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      a.state[1] = 0;
+    if (threadIdx.x == 0) {
       if (a.fail) atomicOr(a.fail, kFailBarrier);
+      if (blockIdx.x == 0) a.state[1] = 0;
     }
     return false;
   };

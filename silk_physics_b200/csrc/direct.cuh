@@ -54,6 +54,7 @@ struct DirectArgs {
   const float* rel_tol_dev = nullptr;
   float rel_tol = 1e-3f, abs_tol = 1e-7f;
   long long barrier_spin_limit = 0;
+  int withhold_block = -1;  // >= 0: that block skips its barrier arrivals (tests)
 };
 
 // One level of the factorisation.

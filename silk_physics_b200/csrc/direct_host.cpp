@@ -299,6 +299,7 @@ void DirectSystem::solve(const CgArgs& cg, cudaStream_t st) {
   a.rel_tol = cg.rel_tol;
   a.abs_tol = cg.abs_tol;
   a.barrier_spin_limit = cg.barrier_spin_limit;
+  a.withhold_block = cg.withhold_block;
   launch_direct_solve(a, blocks_, smem_, st);
 }
 

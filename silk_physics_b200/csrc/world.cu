@@ -1483,7 +1483,7 @@ silk_status World::solver_step() {
         int f = 0;
         CUDA_CHECK(cudaMemcpy(&f, cg_fail.p, sizeof(int), cudaMemcpyDeviceToHost));
         last_error = (f & kFailMasPivot) ? "MAS bank inverse failed: zero or non-finite pivot"
-                     : (f & kFailBarrier) ? "CG barrier wait gave up"
+                     : (f & kFailBarrier) ? "CG or direct solve barrier wait gave up"
                      : (f & kFailContactWait) ? "contact Gauss-Seidel wait gave up"
                      : (f & kFailMlpWait) ? "learned warm start tensor-core wait gave up"
                                           : "solver diverged";

@@ -172,8 +172,8 @@ class SolverOptions:
     contact_gs_form: int = 0          # 0: single-block Gauss-Seidel where possible; 1: grid
     admm_extrapolated_start: bool = False  # offer 2 x_k - x_(k-1) as later CG starts
     resident_halo_limit: int = 0  # > 0: fewer halo slots per resident-CG block (0: 1024)
-    barrier_spin_limit: int = 0  # > 0: polls before a CG grid-barrier wait gives up
-    debug_withhold_block: int = 0  # k > 0: block k - 1 of a cooperative CG grid never arrives
+    barrier_spin_limit: int = 0  # > 0: polls before a grid-barrier wait gives up
+    debug_withhold_block: int = 0  # k > 0: block k - 1 of a cooperative CG grid or direct solve never arrives
     admm_check_interval: int = 0  # ADMM iterations between host reads of the device's convergence state (0: 4)
 
     def to_c(self) -> _SolverOptionsC:

@@ -120,3 +120,31 @@ def test_direct_form_on_every_device():
             assert w.get_cloth_position(h, x)
             out.append(x)
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("block", [1, 2])
+def test_direct_barrier_wait_runs_out(block):
+    """A direct solve in which one block never arrives at its barriers (test
+    switch debug_withhold_block; the CG before it runs as one cluster, whose
+    barrier the switch does not reach): the bounded waits end, the step
+    reports IterativeSolveFail, and the world steps normally afterwards."""
+    V, F = S.grid_sheet(60, jitter=1e-4, seed=3)
+    w = N.World()
+    assert w.init()
+    assert w.set_global_config(N.GlobalConfig(max_inner_iteration=24, admm_abs_tol=0.0,
+                                              admm_rel_tol=0.0))
+    r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+        is_collision_on=False, is_self_collision_on=False), V, F, S.top_corner_pins(60))
+    assert r
+    assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5,
+                                                barrier_spin_limit=1 << 16,
+                                                debug_withhold_block=block))
+    r = w.solver_step()
+    assert r.code == N.ErrorCode.IterativeSolveFail, r.to_string()
+    assert "barrier" in r.detail, r.detail
+    assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5))
+    assert w.set_cloth_state(h, V)
+    r = w.solver_step()
+    assert r, r.to_string()
+    st = w.step_stats()
+    assert st.admm_iterations == 24 and st.cg_solves == DIRECT_FROM - 1
