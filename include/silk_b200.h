@@ -200,6 +200,22 @@ typedef struct {
                                   from the iterate model's prediction */
 } silk_step_stats;
 
+/* The direct form of long ADMM solves (silk_solver_options.cg_form 0) over the
+ * last solver_step, all cloths together; zeros where no solve reached it. */
+typedef struct {
+  int32_t first_iteration; /* ADMM iteration from which the systems of a solve
+                              go to it (a constant of the library) */
+  int32_t factorisations;
+  int32_t solves;          /* systems it solved */
+  int32_t misses;          /* systems whose tolerance it could not meet: solved
+                              by the CG from their own start, and counted there */
+  int32_t applications;    /* of the factors, by solves and misses together */
+  int32_t reserved;
+  double application_bytes; /* compulsory DRAM bytes of those applications */
+  double factor_ms;        /* events (silk_solver_options.profile): factorisations */
+  double solve_ms;         /* events: its solves (part of admm_other_ms too) */
+} silk_direct_stats;
+
 /* --- World lifetime (silk.hpp:92-100) ---------------------------------- */
 silk_world* silk_world_create(void);
 void silk_world_destroy(silk_world* w);
@@ -261,6 +277,7 @@ silk_status silk_set_obstacle_position(silk_world* w, uint32_t handle,
 void silk_solver_options_default(silk_solver_options* o);
 silk_status silk_set_solver_options(silk_world* w, const silk_solver_options* o);
 silk_status silk_get_step_stats(const silk_world* w, silk_step_stats* s);
+silk_status silk_get_direct_stats(const silk_world* w, silk_direct_stats* s);
 /* Launch all device work of this world on the given cudaStream_t (NULL =
  * the world's own stream).  Lets a caller time steps with its own events. */
 silk_status silk_set_stream(silk_world* w, void* cuda_stream);

@@ -234,6 +234,13 @@ silk_status silk_get_step_stats(const silk_world* w, silk_step_stats* s) {
   return SILK_OK;
 }
 
+silk_status silk_get_direct_stats(const silk_world* w, silk_direct_stats* s) {
+  if (!w || !s) return SILK_ERR_INVALID_CONFIG;
+  *s = w->impl.direct_stats;
+  s->first_iteration = silkb::kDirectFrom;
+  return SILK_OK;
+}
+
 silk_status silk_set_stream(silk_world* w, void* cuda_stream) {
   return guard_init(w, [&](World& W) { return W.set_stream(cuda_stream); });
 }

@@ -39,8 +39,8 @@ __device__ __forceinline__ long long up(int N, int i, int j) {
 
 __global__ void direct_begin_kernel(int* state, unsigned* barrier, const int* skip) {
   if (skip && *skip) return;
-  state[0] = 0;
-  state[1] = 0;
+  state[kDirectFailed] = 0;
+  state[kDirectSolved] = 0;
   barrier[0] = barrier[1] = barrier[2] = 0;
 }
 
@@ -536,8 +536,8 @@ __device__ double direct_residual(const DirectArgs& a, bool first, bool second) 
 
 __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectArgs a) {
   if (a.skip && *a.skip) return;  // the ADMM solve already ended (every block alike)
-  if (a.state[0] != 0) {          // no factorisation (every block alike)
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.state[1] = 0;
+  if (a.state[kDirectFailed] != 0) {  // no factors (every block alike)
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.state[kDirectSolved] = 0;
     return;
   }
   extern __shared__ float4 sm[];
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
     if (bar.sync()) return true;
     if (threadIdx.x == 0) {
       if (a.fail) atomicOr(a.fail, kFailBarrier);
-      if (blockIdx.x == 0) a.state[1] = 0;
+      if (blockIdx.x == 0) a.state[kDirectSolved] = 0;
     }
     return false;
   };
@@ -564,7 +564,8 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
   const double rr0 = grid_total(a.partials, gridDim.x);
   double rr = rr0;
   bool ok = false;
-  for (int app = 0; app < kDirectMaxApplications; ++app) {
+  int app = 0;
+  while (app < kDirectMaxApplications) {
     for (int l = a.levels - 1; l > 0; --l) {
       direct_level<true>(a, a.fwd[l], false, sm);
       if (!sync()) return;
@@ -574,7 +575,8 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
       if (!sync()) return;
     }
     p = block_total(direct_residual(a, false, app == 0));
-    double* part = a.partials + (size_t)((app + 1) & 1) * gridDim.x;
+    ++app;
+    double* part = a.partials + (size_t)(app & 1) * gridDim.x;
     if (threadIdx.x == 0) part[blockIdx.x] = p;
     if (!sync()) return;
     const double now = grid_total(part, gridDim.x);
@@ -585,7 +587,11 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
   // The last block to leave clears the barrier for the next solve.
   if (threadIdx.x == 0 && atomicAdd(a.barrier + 2, 1u) == gridDim.x - 1)
     a.barrier[0] = a.barrier[2] = 0u;
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.state[1] = ok ? 1 : 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.state[kDirectSolved] = ok ? 1 : 0;
+    a.state[ok ? kDirectSolves : kDirectMisses] += 1;
+    a.state[kDirectApplied] += app;
+  }
   if (!ok) return;  // the CG launched after this solves from the unchanged start
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nv; i += gridDim.x * blockDim.x)
     a.x[i] = __ldcg(a.xn + i);

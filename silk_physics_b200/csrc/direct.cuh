@@ -25,6 +25,16 @@ constexpr int kDirectMaxLevels = 12;
 constexpr int kDirectThreads = 1024;
 constexpr int kDirectMaxApplications = 4;
 
+// Words of DirectArgs::state.  The last three count over a step.
+enum DirectState {
+  kDirectFailed = 0,    // no usable factors
+  kDirectSolved = 1,    // the last solve met its tolerance
+  kDirectSolves = 2,    // solves that met it
+  kDirectMisses = 3,    // solves that did not (left to the CG)
+  kDirectApplied = 4,   // applications of the factors
+  kDirectWords = 5
+};
+
 struct DirectArgs {
   int nv = 0, nslices = 0, levels = 0;
   const int* sl_ptr = nullptr;
@@ -48,7 +58,7 @@ struct DirectArgs {
   float4* xn = nullptr;   // x plus the corrections so far
   double* partials = nullptr;
   unsigned* barrier = nullptr;  // [count, err, blocks that left]
-  int* state = nullptr;  // [0] factorisation failed, [1] this solve met its tolerance
+  int* state = nullptr;  // kDirectWords words
   int* fail = nullptr;   // kFail* word of the solver
   const int* skip = nullptr;
   const float* rel_tol_dev = nullptr;

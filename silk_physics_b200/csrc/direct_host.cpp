@@ -166,6 +166,10 @@ DirectSystem::DirectSystem(const ClothSetup& S, const std::vector<float>& rest,
     arena_.reset();
     return;
   }
+  // Factors; 8 B per entry of L and 16 B per vertex for dx, r, xn (read and
+  // written), Ldiag and dyn.
+  application_bytes_ = 4.0 * (double)(P.g_total + P.t_total) +
+                       8.0 * (double)(S.Lcols.size() - (size_t)S.nv) + (5 * 16.0 + 8.0) * S.nv;
   args_.nv = S.nv;
   args_.levels = nl;
   args_.nodes = nodes_;
@@ -221,7 +225,7 @@ void DirectSystem::upload(const DirectPlan& P, const std::vector<DirectNodeDev>&
     for (float4** v : {&f_, &r_, &dx_, &xn_}) place(*v, nv);
     place(partials_, 2 * (size_t)blocks_);
     place(barrier_, 3);
-    place(state_, 2);
+    place(state_, kDirectWords);
     if (pass == 0) {
       arena_.alloc(need);
       base = arena_.p;
@@ -242,7 +246,14 @@ void DirectSystem::upload(const DirectPlan& P, const std::vector<DirectNodeDev>&
   copy(diag_dst_, P.diag_dst);
   copy(tasks_, tasks);
   copy(lists_, lists);
-  CUDA_CHECK(cudaMemsetAsync(state_, 0, 2 * sizeof(int), st));
+  CUDA_CHECK(cudaMemsetAsync(state_, 0, kDirectWords * sizeof(int), st));
+}
+
+void DirectSystem::begin_step(cudaStream_t st) {
+  factorisations_ = 0;
+  if (usable_)
+    CUDA_CHECK(cudaMemsetAsync(state_ + kDirectSolves, 0,
+                               (kDirectWords - kDirectSolves) * sizeof(int), st));
 }
 
 void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* skip,
@@ -265,6 +276,7 @@ void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* s
   a.T = T_;
   a.state = state_;
   a.skip = skip;
+  ++factorisations_;
   launch_direct_begin(state_, barrier_, skip, st);
   for (int l = (int)levels_.size() - 1; l >= 0; --l) {
     const Level& L = levels_[l];

@@ -18,7 +18,15 @@ class DirectSystem {
   // Solves into a.x, to the tolerance of the CG solve `cg` stands for.
   void solve(const CgArgs& cg, cudaStream_t st);
   // Set when the last solve met its tolerance (the CG then has nothing to do).
-  const int* solved() const { return state_ + 1; }
+  const int* solved() const { return state_ + kDirectSolved; }
+  // Counts over a step: cleared on `st`, read from state() (kDirectWords
+  // words on the device).
+  void begin_step(cudaStream_t st);
+  const int* state() const { return state_; }
+  int factorisations() const { return factorisations_; }
+  // Compulsory DRAM bytes of one application: the factors once, the matrix
+  // rows and the vectors of its residual.
+  double application_bytes() const { return application_bytes_; }
 
  private:
   struct Level {
@@ -36,8 +44,9 @@ class DirectSystem {
               cudaStream_t st);
 
   bool usable_ = false;
-  int blocks_ = 0;
+  int blocks_ = 0, factorisations_ = 0;
   size_t smem_ = 0;
+  double application_bytes_ = 0.0;
   std::vector<Level> levels_;
   DirectArgs args_;
   // Everything on the device, in one allocation.

@@ -29,13 +29,6 @@ struct NvtxRange {
 
 namespace {
 
-// ADMM iteration from which a solve's systems go to the direct form, and with
-// them those of every later ADMM solve of the step.  A factorisation costs
-// about four CG solves (0.9 ms against 0.24 at 6,400 vertices, 6.5 against
-// 1.7 at 100K), so short solves stay with the CG; one that has come this far
-// is likely to take as many iterations again.
-constexpr int kDirectFrom = 16;
-
 std::vector<float4> to_float4(const std::vector<float>& v3, const std::vector<int>& perm) {
   int n = (int)perm.size();
   std::vector<float4> out(n);
@@ -53,7 +46,7 @@ World::World() {
 
 World::~World() {
   coll_.reset();
-  for (auto* pool : {&events, &events_other, &events_gs})
+  for (auto* pool : {&events, &events_other, &events_gs, &events_factor, &events_direct})
     for (auto& e : *pool) {
       cudaEventDestroy(e.first);
       cudaEventDestroy(e.second);
@@ -1087,7 +1080,10 @@ void World::cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStrea
   if (direct && c.dev.direct->usable()) {
     auto* ev = opt.profile ? next_event_pair(events_other, events_other_used) : nullptr;
     if (ev) CUDA_CHECK(cudaEventRecord(ev->first, st));
+    auto* dv = opt.profile ? next_event_pair(events_direct, events_direct_used) : nullptr;
+    if (dv) CUDA_CHECK(cudaEventRecord(dv->first, st));
     c.dev.direct->solve(a, st);
+    if (dv) CUDA_CHECK(cudaEventRecord(dv->second, st));
     a.solved = c.dev.direct->solved();
     launch();
     if (ev) CUDA_CHECK(cudaEventRecord(ev->second, st));
@@ -1347,8 +1343,12 @@ bool World::admm_solve() {
         if (direct && !factored) {
           if (!c.dev.direct)
             c.dev.direct = std::make_shared<DirectSystem>(*c.setup, c.rest, cs);
-          if (c.dev.direct->usable())
+          if (c.dev.direct->usable()) {
+            auto* fv = opt.profile ? next_event_pair(events_factor, events_factor_used) : nullptr;
+            if (fv) CUDA_CHECK(cudaEventRecord(fv->first, cs));
             c.dev.direct->factorize(c.dev.Lvals.p, lhs.p + c.voff, done, cs);
+            if (fv) CUDA_CHECK(cudaEventRecord(fv->second, cs));
+          }
         }
         cg_solve(c, rel, it == 1, direct, cs);
         if (cs != st) {
@@ -1408,6 +1408,7 @@ silk_status World::solver_step() {
     };
     auto t_step = clk::now();
     stats = silk_step_stats{};
+    direct_stats = silk_direct_stats{};
     step_direct_ = false;
     if (cloths.empty()) {
       last_error = "nothing to solve";
@@ -1417,8 +1418,13 @@ silk_status World::solver_step() {
     upload_pins();
     cudaStream_t st = stream;
     int nv = nv_total;
-    for (auto& c : cloths) c->dev.stats.zero(st);
+    for (auto& c : cloths) {
+      c->dev.stats.zero(st);
+      if (c->dev.direct) c->dev.direct->begin_step(st);
+    }
     events_used = 0;
+    events_factor_used = 0;
+    events_direct_used = 0;
     events_other_used = 0;
     events_gs_used = 0;
     CUDA_CHECK(cudaMemcpyAsync(step_start.p, sx.p, nv * sizeof(float4), cudaMemcpyDeviceToDevice, st));
@@ -1536,6 +1542,13 @@ silk_status World::solver_step() {
     for (size_t k = 0; k < cloths.size(); ++k)
       CUDA_CHECK(cudaMemcpyAsync(&cgs[kCgStats * k], cloths[k]->dev.stats.p,
                                  kCgStats * sizeof(int), cudaMemcpyDeviceToHost, st));
+    std::vector<int> direct(kDirectWords * cloths.size(), 0);
+    for (size_t k = 0; k < cloths.size(); ++k) {
+      const DirectSystem* d = cloths[k]->dev.direct.get();
+      if (d && d->factorisations() > 0)
+        CUDA_CHECK(cudaMemcpyAsync(&direct[kDirectWords * k], d->state(),
+                                   kDirectWords * sizeof(int), cudaMemcpyDeviceToHost, st));
+    }
     sync();
     for (size_t k = 0; k < cloths.size(); ++k) {
       const int* q = &cgs[kCgStats * k];
@@ -1548,6 +1561,14 @@ silk_status World::solver_step() {
       stats.learned_starts += q[3];
       stats.extrapolated_starts += q[4];
       stats.learned_iterate_starts += q[5];
+      if (const DirectSystem* d = cloths[k]->dev.direct.get()) {
+        const int* s = &direct[kDirectWords * k];
+        direct_stats.factorisations += d->factorisations();
+        direct_stats.solves += s[kDirectSolves];
+        direct_stats.misses += s[kDirectMisses];
+        direct_stats.applications += s[kDirectApplied];
+        direct_stats.application_bytes += s[kDirectApplied] * d->application_bytes();
+      }
       if (opt.profile) {
         double bpi = opt.mas_bf16 ? cloths[k]->dev.bytes_per_iter_bf16
                                   : cloths[k]->dev.bytes_per_iter_fp32;
@@ -1564,6 +1585,16 @@ silk_status World::solver_step() {
       // Solves that ran (launches of iterations enqueued after the ADMM
       // solve ended return at entry; their events add a few us).
       for (size_t k = 0; k < cloths.size(); ++k) prof.cg_launches += cgs[kCgStats * k + 1];
+      for (size_t e = 0; e < events_factor_used; ++e) {
+        float ms = 0.f;
+        CUDA_CHECK(cudaEventElapsedTime(&ms, events_factor[e].first, events_factor[e].second));
+        direct_stats.factor_ms += ms;
+      }
+      for (size_t e = 0; e < events_direct_used; ++e) {
+        float ms = 0.f;
+        CUDA_CHECK(cudaEventElapsedTime(&ms, events_direct[e].first, events_direct[e].second));
+        direct_stats.solve_ms += ms;
+      }
       for (size_t e = 0; e < events_gs_used; ++e) {
         float ms = 0.f;
         CUDA_CHECK(cudaEventElapsedTime(&ms, events_gs[e].first, events_gs[e].second));

@@ -215,6 +215,13 @@ class StepStats:
     learned_iterate_starts: int = 0
 
 
+class _DirectStatsC(C.Structure):
+    _fields_ = [("first_iteration", C.c_int32), ("factorisations", C.c_int32),
+                ("solves", C.c_int32), ("misses", C.c_int32), ("applications", C.c_int32),
+                ("reserved", C.c_int32), ("application_bytes", C.c_double),
+                ("factor_ms", C.c_double), ("solve_ms", C.c_double)]
+
+
 _F32P = np.ctypeslib.ndpointer(np.float32, flags="C_CONTIGUOUS")
 _I32P = np.ctypeslib.ndpointer(np.int32, flags="C_CONTIGUOUS")
 _F64P = np.ctypeslib.ndpointer(np.float64, flags="C_CONTIGUOUS")
@@ -259,6 +266,7 @@ def _load() -> C.CDLL:
         "silk_set_solver_options": ([_W, C.POINTER(_SolverOptionsC)], C.c_int),
         "silk_get_step_stats": ([_W, C.POINTER(_StepStatsC)], C.c_int),
         "silk_set_stream": ([_W, C.c_void_p], C.c_int),
+        "silk_get_direct_stats": ([_W, C.POINTER(_DirectStatsC)], C.c_int),
         "silk_get_profile": ([_W, C.POINTER(_ProfileC), C.c_int32], C.c_int),
         "silk_get_cloth_velocity": ([_W, C.c_uint32, _F32P, C.c_int64], C.c_int),
         "silk_set_cloth_state": ([_W, C.c_uint32, _F32P, C.c_int64, C.c_void_p, C.c_int64],
@@ -438,6 +446,13 @@ class World:
         s = _StepStatsC()
         lib.silk_get_step_stats(self._w, C.byref(s))
         return StepStats(**{n: getattr(s, n) for n in StepStats.__dataclass_fields__})
+
+    def direct_stats(self) -> dict:
+        """The direct form over the last step: factorisations, systems solved
+        and missed, applications, and with profile their event times."""
+        s = _DirectStatsC()
+        lib.silk_get_direct_stats(self._w, C.byref(s))
+        return {n: getattr(s, n) for n, _ in _DirectStatsC._fields_ if n != "reserved"}
 
     def set_stream(self, cuda_stream: int | None) -> Result:
         return _result(lib.silk_set_stream(self._w, cuda_stream or None), self._w)

@@ -148,3 +148,30 @@ def test_direct_barrier_wait_runs_out(block):
     assert r, r.to_string()
     st = w.step_stats()
     assert st.admm_iterations == 24 and st.cg_solves == DIRECT_FROM - 1
+
+
+def test_direct_form_is_counted():
+    """What the direct form did in a step: every system from the threshold on
+    is counted as solved or missed, with its factorisations, applications and
+    event times; a step without it counts nothing."""
+    V, F = S.grid_sheet(40, jitter=1e-4, seed=3)
+    w = N.World()
+    assert w.init()
+    r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+        is_collision_on=False, is_self_collision_on=False), V, F, S.top_corner_pins(40))
+    assert r
+    for inner, form in ((24, 0), (DIRECT_FROM, 0), (24, 3), (24, 0)):
+        assert w.set_global_config(N.GlobalConfig(max_inner_iteration=inner, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5, cg_form=form,
+                                                    profile=1))
+        assert w.solver_step()
+        st, d = w.step_stats(), w.direct_stats()
+        direct = inner - DIRECT_FROM if form == 0 else 0
+        assert d["first_iteration"] == DIRECT_FROM
+        assert d["solves"] == direct and d["misses"] == 0
+        assert st.cg_solves == inner - 1 - direct
+        assert d["factorisations"] == (1 if direct else 0)
+        assert direct <= d["applications"] <= 4 * direct
+        for key in ("application_bytes", "factor_ms", "solve_ms"):
+            assert (d[key] > 0) == (direct > 0)
