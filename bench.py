@@ -50,6 +50,7 @@ C3_WORKLOAD = "c3_sheet316_on_icosphere_r0.6_first_contact"
 STATE = ROOT / "oracle" / "reference_state_c2_step27.npz"
 MODEL = ROOT / "silk_physics_b200" / "models" / "warm_start.npy"
 TRAFFIC = ROOT / "profiles" / "cg_cluster_c2_contact.json"
+TRAFFIC_DIRECT = ROOT / "profiles" / "direct_solve_c2_contact.json"
 SCENES = ROOT / "tests" / "golden" / "reference_scenes.npz"
 C3_START_STEPS = 8  # free-fall steps before the drape's first contact step
 
@@ -201,14 +202,12 @@ def peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
-def traffic_per_launch():
-    """DRAM bytes per CG launch of a contact-regime solve, from the committed
-    ncu summary (profiles/cg_cluster_c2_contact.json), or None."""
-    if not TRAFFIC.exists():
-        return None
-    d = json.loads(TRAFFIC.read_text())
-    return {"bytes": d["dram_bytes_per_launch"], "source": TRAFFIC.name,
-            "captured": d.get("captured")}
+def traffic_per_launch(path):
+    """Traffic fields of a roofline entry: DRAM bytes per launch of a
+    contact-regime solve, from a committed ncu summary (None without it)."""
+    d = json.loads(path.read_text()) if path.exists() else {}
+    return {"traffic": d.get("dram_bytes_per_launch"),
+            "traffic_source": f"{path.name}: {d.get('captured')}" if d else None}
 
 
 def make_world(stream_handle, opts, V, F, SV, SF, model=False):
@@ -283,7 +282,7 @@ def replay_variant(N, torch, stream, flush, V, F, SV, SF, x0, v0, cg_rel_tol, bf
         ms.append(a.elapsed_time(b))
         s = w.step_stats()
         keys.add((s.admm_iterations, s.cg_iterations, s.contacts, s.outer_iterations))
-    s = w.step_stats()
+    s, d = w.step_stats(), w.direct_stats()
     prof = w.profile(reset=True)
     med = statistics.median(ms)
     return {"ms_per_step_median": round(med, 2), "ms_per_step": [round(t, 2) for t in ms],
@@ -295,6 +294,9 @@ def replay_variant(N, torch, stream, flush, V, F, SV, SF, x0, v0, cg_rel_tol, bf
             "first_solve_cg_iterations": s.cg_first_solve_iterations,
             "ms_per_admm_iteration": round(med / max(s.admm_iterations, 1), 4),
             "cg_kernel_ms_per_step": round(prof["cg_time_ms"] / reps, 2),
+            "direct_solves_per_step": d["solves"], "direct_misses_per_step": d["misses"],
+            "direct_solve_ms_per_step": round(d["solve_ms"], 2),
+            "direct_factor_ms_per_step": round(d["factor_ms"], 2),
             "contact_gs_ms_per_step": round(prof["contact_gs_ms"] / reps, 2),
             "ccd_host_ms_per_step": round(prof["ccd_host_ms"] / reps, 2),
             "ccd_refit_host_ms_per_step": round(prof["ccd_refit_host_ms"] / reps, 2),
@@ -456,6 +458,8 @@ def run_ours(args) -> None:
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
           for _ in range(args.steps)]
     launches = admm = cg = solves = contacts = cluster_solves = 0
+    direct = dict(factorisations=0, solves=0, misses=0, applications=0, application_bytes=0.0,
+                  factor_ms=0.0, solve_ms=0.0)
     per_step_admm = []
     if world_size > 1:
         torch.distributed.barrier()
@@ -476,6 +480,8 @@ def run_ours(args) -> None:
             solves += st.cg_solves
             cluster_solves += st.cg_cluster_solves
             contacts = st.contacts
+            ds = w.direct_stats()
+            direct = {key: direct[key] + ds[key] for key in direct}
         torch.cuda.synchronize()
     step_ms = [a.elapsed_time(b) for a, b in ev]
     total_ms = float(sum(step_ms))
@@ -523,19 +529,34 @@ def run_ours(args) -> None:
     cg_launch_ms = prof["cg_time_ms"] / max(prof["cg_launches"], 1)
     bytes_per_launch = prof["cg_algorithmic_bytes"] / max(prof["cg_launches"], 1)
     achieved = bytes_per_launch / (cg_launch_ms / 1e3) / 1e9 if cg_launch_ms > 0 else 0.0
-    tr = traffic_per_launch()
     kernel = ("cg_dsm_cluster_kernel (persistent MAS-PCG, cluster form)"
               if cluster_solves == solves else "cg_resident / cg_kernel (persistent MAS-PCG)")
     roofline = {"bound": "hbm", "kernel": kernel,
                 "achieved": round(achieved, 2), "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": round(achieved / pk["hbm_gbs"], 5), "peak_source": pk["source"],
-                "traffic": tr["bytes"] if tr else None,
-                "traffic_source": (f"{tr['source']}: {tr['captured']}" if tr else None),
-                "algorithmic_bytes_per_launch": round(bytes_per_launch),
+                **traffic_per_launch(TRAFFIC), "algorithmic_bytes_per_launch": round(bytes_per_launch),
                 "avg_launch_ms": round(cg_launch_ms, 5),
                 "cg_iterations_per_launch": round(prof["cg_iterations"] /
                                                   max(prof["cg_launches"], 1), 2),
                 "cg_share_of_step": round(prof["cg_time_ms"] / total_ms, 4) if total_ms else None}
+    # The solver kernel that takes more of the step leads; the other one stays
+    # beside it.
+    roofline_other = None
+    if direct["solve_ms"] > 0:
+        tried = direct["solves"] + direct["misses"]
+        got = direct["application_bytes"] / (direct["solve_ms"] / 1e3) / 1e9
+        roofline_other = {"bound": "hbm", "kernel": "direct_solve_kernel (direct form of long "
+                          "ADMM solves)", "achieved": round(got, 2), "peak": pk["hbm_gbs"],
+                          "unit": "GB/s", "frac": round(got / pk["hbm_gbs"], 5),
+                          "peak_source": pk["source"], **traffic_per_launch(TRAFFIC_DIRECT),
+                          "algorithmic_bytes_per_launch":
+                              round(direct["application_bytes"] / max(tried, 1)),
+                          "avg_launch_ms": round(direct["solve_ms"] / max(tried, 1), 5),
+                          "applications_per_launch":
+                              round(direct["applications"] / max(tried, 1), 2),
+                          "share_of_step": round(direct["solve_ms"] / total_ms, 4)}
+        if direct["solve_ms"] > prof["cg_time_ms"]:
+            roofline, roofline_other = roofline_other, roofline
     cpu = None
     if world_size == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
@@ -557,8 +578,12 @@ def run_ours(args) -> None:
         "stats": {"admm_iterations_per_step": admm / args.steps,
                   "admm_iterations_per_timed_step": per_step_admm,
                   "cg_iterations_per_solve": round(cg / max(solves, 1), 2),
+                  "cg_solves_per_step": solves / args.steps,
+                  "direct_per_step": {key: round(direct[key] / args.steps, 2)
+                                      for key in ("factorisations", "solves", "misses",
+                                                  "applications")},
                   "contacts_last_step": contacts},
-        "roofline": roofline, "cpu_baseline": cpu,
+        "roofline": roofline, "roofline_other": roofline_other, "cpu_baseline": cpu,
         "e2e": {"value": round(e2e_val, 4), "unit": "steps/s",
                 "h2d_bytes_per_step": int(SV.nbytes), "d2h_bytes_per_step": int(V.nbytes),
                 "steps": args.steps, "admm_iterations_per_step": e2e_admm,
@@ -577,6 +602,8 @@ def run_ours(args) -> None:
             "cg_kernel_events": round(prof["cg_time_ms"] / args.steps, 2),
             "other_admm_kernels_events": round(prof["admm_other_ms"] / args.steps, 2),
             "contact_gs_events": round(prof["contact_gs_ms"] / args.steps, 2),
+            "direct_solve_events": round(direct["solve_ms"] / args.steps, 2),
+            "direct_factor_events": round(direct["factor_ms"] / args.steps, 2),
             "admm_host_wall": round(prof["admm_host_ms"] / args.steps, 2),
             "ccd_host_wall": round(prof["ccd_host_ms"] / args.steps, 2),
             "dcd_host_wall": round(prof["dcd_host_ms"] / args.steps, 2),
