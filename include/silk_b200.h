@@ -112,7 +112,9 @@ typedef struct {
                                  bit 2: record iterate-model training samples
                                  (256 vertices per ADMM iteration) */
   int32_t contact_gs_form;    /* 0: single-block contact Gauss-Seidel where the
-                                 contacts fit it, else grid; 1: grid always */
+                                 contacts fit it and it is the faster one (up
+                                 to 1,700 contacts a colour), else grid;
+                                 1: grid always */
   int32_t admm_extrapolated_start; /* 1: offer 2 x_k - x_(k-1) (the last two ADMM
                                  iterates of the same ADMM solve) as the start
                                  of each later CG solve; the plain start's

@@ -1464,6 +1464,7 @@ __global__ void contact_gs_kernel(const ContactDev* contacts, const int* groups,
 constexpr int kGsFlowWarps = 12;
 constexpr size_t kGsBlockSmemMax = 226 * 1024;
 constexpr int kGsWaitSpins = 1 << 20;  // polls before a contact gives up
+constexpr int kGsContactsPerColour = 1700;  // more of them go to the grid form
 
 struct GsContact {
   int slot[4];  // compact vertex slot, -1 kinematic
@@ -2551,10 +2552,17 @@ void CollisionSystem::contact_solve_launch() {
   if (I.n_contacts == 0) return;
   cudaStream_t st = w_.stream;
   // Single-block form while the touched vertices' positions fit the block's
-  // shared memory, with the corrections too where they also fit.
+  // shared memory, with the corrections too where they also fit, and while it
+  // is the faster one: with many contacts it is bound by the block's own rate,
+  // about 26 ns a contact and call, the grid form by its colour barriers,
+  // about 45 us a colour and call, so the line lies at 1,700 contacts a colour
+  // (us a call, single-block against grid: 1,607 and 2,863 for 61,692 contacts
+  // in 66 colours, 2,543 and 2,870 for 100,043 in 63, 3,710 and 3,041 for
+  // 142,909 in 65, 6,438 and 5,762 for 246,800 in 114).
   const size_t pos = (size_t)(I.gs_nslots + 1) * sizeof(float4);
   const size_t both = pos + (size_t)I.n_contacts * sizeof(float4);
-  if (I.gs_ready && w_.opt.contact_gs_form != 1 && pos <= kGsBlockSmemMax) {
+  if (I.gs_ready && w_.opt.contact_gs_form != 1 && pos <= kGsBlockSmemMax &&
+      I.n_contacts <= kGsContactsPerColour * I.n_colors) {
     static PerDevice<bool> opted;
     opted.get(current_device(), [] {
       for (auto* k : {contact_gs_flow_kernel<true>, contact_gs_flow_kernel<false>})

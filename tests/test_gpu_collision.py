@@ -337,6 +337,43 @@ def test_gs_single_block_sizes_identical(s, so, few, many):
     np.testing.assert_array_equal(out[0][0], out[1][0])
 
 
+@pytest.mark.parametrize("s", [60, 118])
+def test_gs_form_chosen_is_the_faster(s):
+    """Many contacts per colour (about 560 and 2,200): the form that is chosen
+    takes no longer than the grid form (event times of one step, the better of
+    three, 10 % for their spread), and both move every vertex alike."""
+    out = []
+    for form in (0, 1):
+        V, F = S.grid_sheet(s, side=0.5 * (s - 1) / 77, z=1.0, jitter=1e-6, seed=4)
+        OV, OF = S.grid_sheet(s, side=0.52 * (s - 1) / 77, z=0.0)
+        OV[:, 2] = V[:, 2].min() - 0.3 * 0.05 * 0.5 / 77
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(acceleration_z=-9.81, max_inner_iteration=8,
+                                                  max_outer_iteration=1, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-5, profile=1,
+                                                    contact_gs_form=form))
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(is_self_collision_on=False), V, F,
+                           [])
+        r2, _ = w.add_obstacle(N.CollisionConfig(), OV, OF)
+        assert r and r2
+        ms = []
+        for _ in range(3):
+            assert w.set_cloth_state(h, V)
+            w.profile(reset=True)
+            assert w.solver_step()
+            ms.append(w.profile()["contact_gs_ms"])
+        x = np.zeros(V.size, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append((x, min(ms), w.step_stats()))
+    print(f"{s}: {out[0][2].contacts} contacts, {out[0][2].colors} colours, "
+          f"{out[0][1]:.2f} ms, grid {out[1][1]:.2f} ms")
+    assert out[0][2].contacts > 14464
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    assert out[0][1] <= 1.1 * out[1][1]
+
+
 # Pending-box stores of the deep searches: 96 per thread in the first pass,
 # heaps in shared memory (up to about 7,200 boxes), sorted arrays in global
 # memory above that; the smallest cap, around the first pass's size, and both
