@@ -591,6 +591,9 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
     a.state[kDirectSolved] = ok ? 1 : 0;
     a.state[ok ? kDirectSolves : kDirectMisses] += 1;
     a.state[kDirectApplied] += app;
+    // Given up once it has missed more often than not in this step: the
+    // tries then cost no more than the solves before them have saved.
+    if (!ok && a.state[kDirectMisses] > a.state[kDirectSolves]) a.state[kDirectFailed] = 1;
   }
   if (!ok) return;  // the CG launched after this solves from the unchanged start
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nv; i += gridDim.x * blockDim.x)

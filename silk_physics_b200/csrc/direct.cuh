@@ -27,7 +27,7 @@ constexpr int kDirectMaxApplications = 4;
 
 // Words of DirectArgs::state.  The last three count over a step.
 enum DirectState {
-  kDirectFailed = 0,    // no usable factors
+  kDirectFailed = 0,    // no usable factors, or given up
   kDirectSolved = 1,    // the last solve met its tolerance
   kDirectSolves = 2,    // solves that met it
   kDirectMisses = 3,    // solves that did not (left to the CG)

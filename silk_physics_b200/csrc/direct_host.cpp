@@ -251,6 +251,7 @@ void DirectSystem::upload(const DirectPlan& P, const std::vector<DirectNodeDev>&
 
 void DirectSystem::begin_step(cudaStream_t st) {
   factorisations_ = 0;
+  given_up_ = false;
   if (usable_)
     CUDA_CHECK(cudaMemsetAsync(state_ + kDirectSolves, 0,
                                (kDirectWords - kDirectSolves) * sizeof(int), st));

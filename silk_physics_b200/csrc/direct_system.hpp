@@ -12,7 +12,9 @@ class DirectSystem {
   // Builds the plan and its device arrays on `st`.  usable() is false when
   // the fronts would not pay or do not fit the device's free memory.
   DirectSystem(const ClothSetup& S, const std::vector<float>& rest, cudaStream_t st);
-  bool usable() const { return usable_; }
+  // Nor is it after give_up(), until the next step.
+  bool usable() const { return usable_ && !given_up_; }
+  void give_up() { given_up_ = true; }
   // Factorises L + diag(dyn) (kernels return at entry once *skip is set).
   void factorize(const double* Lvals, const float* dyn, const int* skip, cudaStream_t st);
   // Solves into a.x, to the tolerance of the CG solve `cg` stands for.
@@ -43,7 +45,7 @@ class DirectSystem {
               const int64_t (&front)[2], int64_t gd, int panel, int level_nodes, int nv,
               cudaStream_t st);
 
-  bool usable_ = false;
+  bool usable_ = false, given_up_ = false;
   int blocks_ = 0, factorisations_ = 0;
   size_t smem_ = 0;
   double application_bytes_ = 0.0;

@@ -1392,6 +1392,18 @@ bool World::admm_solve() {
   const int ran = enqueued <= 1 ? enqueued : ctl_host_.iteration + 1;
   stats.admm_iterations += ran;
   if (ran > kDirectFrom) step_direct_ = true;
+  // Where the matrix had no factors or the tolerance was out of reach, the
+  // step's later ADMM solves do not factorise for it again.
+  if (factored) {
+    std::vector<int> failed(cloths.size(), 0);
+    for (size_t k = 0; k < cloths.size(); ++k)
+      if (cloths[k]->dev.direct->usable())
+        CUDA_CHECK(cudaMemcpyAsync(&failed[k], cloths[k]->dev.direct->state() + kDirectFailed,
+                                   sizeof(int), cudaMemcpyDeviceToHost, st));
+    sync();
+    for (size_t k = 0; k < cloths.size(); ++k)
+      if (failed[k]) cloths[k]->dev.direct->give_up();
+  }
   if (ctl_host_.diverged) return false;
   launch_enforce(s, st);
   return true;

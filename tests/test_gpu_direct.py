@@ -175,3 +175,38 @@ def test_direct_form_is_counted():
         assert direct <= d["applications"] <= 4 * direct
         for key in ("application_bytes", "factor_ms", "solve_ms"):
             assert (d[key] > 0) == (direct > 0)
+
+
+def test_direct_form_gives_up_on_a_tolerance_out_of_reach():
+    """A sheet landing on a ball at a tolerance that no refinement reaches:
+    one miss ends the tries of its ADMM solve and of the step's later ones,
+    which do not factorise either; the CG form's bits."""
+    V, F = S.grid_sheet(24, side=0.5, z=0.31, jitter=1e-4, seed=3)
+    SV, SF = S.icosphere(2, radius=0.3)
+    out = []
+    for form in (0, 3):
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(max_inner_iteration=24, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0, linear_solver_abs_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-30, cg_form=form,
+                                                    cg_max_iter=40))
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(), V, F, [])
+        assert r
+        r, _ = w.add_obstacle(N.CollisionConfig(), SV, SF)
+        assert r
+        got = []
+        for _ in range(3):
+            r = w.solver_step()
+            assert r, r.to_string()
+            st, d = w.step_stats(), w.direct_stats()
+            got.append((st.outer_iterations, st.cg_solves))
+            assert st.cg_solves == 23 * st.outer_iterations
+            assert (d["factorisations"], d["misses"], d["solves"]) == \
+                ((1, 1, 0) if form == 0 else (0, 0, 0))
+        x = np.zeros(V.size, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append((got, x))
+    assert max(o for o, _ in out[0][0]) > 1
+    assert out[0][0] == out[1][0]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
