@@ -210,3 +210,74 @@ def test_direct_form_gives_up_on_a_tolerance_out_of_reach():
     assert max(o for o, _ in out[0][0]) > 1
     assert out[0][0] == out[1][0]
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+def _two_cloths(form, tol, sizes, over):
+    """Cloths of the given sides, each flat within contact distance of its own
+    plate (over) or free, one ADMM solve of 40 iterations in one world."""
+    w = N.World()
+    assert w.init()
+    assert w.set_global_config(N.GlobalConfig(max_inner_iteration=40, max_outer_iteration=1,
+                                              admm_abs_tol=0.0, admm_rel_tol=0.0,
+                                              linear_solver_abs_tol=0.0))
+    assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=tol, cg_form=form))
+    handles = []
+    for k, s in sizes:
+        V, F = S.grid_sheet(s, side=(s - 1) / 79, z=1.0, jitter=1e-5, seed=k)
+        V[:, 0] += 3.0 * k
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+            is_collision_on=over, is_self_collision_on=False), V, F, [])
+        assert r, r.to_string()
+        handles.append((h, V.size))
+        if over:
+            n = s // 4
+            OV, OF = S.grid_sheet(n, side=1.1 * (s - 1) / 79, z=0.0)
+            OV[:, 0] += 3.0 * k + 0.5 * (V[:, 0].min() + V[:, 0].max() - 6.0 * k) \
+                - 0.5 * (OV[:, 0].min() + OV[:, 0].max())
+            OV[:, 1] += 0.5 * (V[:, 1].min() + V[:, 1].max() - OV[:, 1].min() - OV[:, 1].max())
+            OV[:, 2] = V[:, 2].min() - 2e-4
+            r, _ = w.add_obstacle(N.CollisionConfig(), OV, OF)
+            assert r, r.to_string()
+    r = w.solver_step()
+    assert r, r.to_string()
+    out = []
+    for h, n in handles:
+        x = np.zeros(n, np.float32)
+        assert w.get_cloth_position(h, x)
+        out.append(x.astype(np.float64))
+    return out, w.step_stats(), w.direct_stats()
+
+
+# A CG in one cluster (its own stream) beside a cooperative grid (the world's
+# stream), in both orders, and two clusters side by side.
+TWO = [((0, 24), (1, 136)), ((0, 136), (1, 24)), ((0, 40), (1, 33))]
+
+
+@pytest.mark.parametrize("sizes", TWO)
+def test_two_cloths_are_solved_as_alone(sizes):
+    """Cloths without contact are independent systems: stepped in one world
+    and each in a world of its own they end in the same bits."""
+    both, st, d = _two_cloths(0, 1e-5, sizes, False)
+    assert d["solves"] == 2 * (40 - DIRECT_FROM) and d["misses"] == 0
+    assert st.cg_solves == 2 * (DIRECT_FROM - 1)
+    for x, size in zip(both, sizes):
+        alone, _, _ = _two_cloths(0, 1e-5, [size], False)
+        np.testing.assert_array_equal(x, alone[0])
+
+
+@pytest.mark.parametrize("sizes", TWO)
+def test_two_cloths_in_contact_match_cg(sizes):
+    """Two cloths in contact, the direct form against CG throughout.  Contacts
+    that open or close amplify what a solve leaves and how it is rounded, so
+    the yardstick is the larger distance of two CG forms (solved to 1e-6, sums
+    in other orders) from the CG solved to 1e-8; no absolute tolerance, which
+    would stop all of them alike."""
+    out = [_two_cloths(form, tol, sizes, True) for form, tol in
+           ((0, 1e-6), (3, 1e-6), (1, 1e-6), (3, 1e-8))]
+    assert out[0][2]["solves"] > 0 and out[0][1].contacts > 0
+    assert all(o[1].contacts == out[0][1].contacts for o in out)
+    for k in range(2):
+        err = np.abs(out[0][0][k] - out[3][0][k]).max()
+        own = max(np.abs(o[0][k] - out[3][0][k]).max() for o in out[1:3])
+        print(f"{sizes[k]}: {out[0][1].contacts} contacts, direct {err:.2e}, CG {own:.2e}")
+        assert err <= max(3.0 * own, 5e-6)
