@@ -537,7 +537,10 @@ __device__ double direct_residual(const DirectArgs& a, bool first, bool second) 
 __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectArgs a) {
   if (a.skip && *a.skip) return;  // the ADMM solve already ended (every block alike)
   if (a.state[kDirectFailed] != 0) {  // no factors (every block alike)
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.state[kDirectSolved] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.state[kDirectSolved] = 0;
+      *a.failed = 1;
+    }
     return;
   }
   extern __shared__ float4 sm[];
@@ -589,11 +592,12 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
     a.barrier[0] = a.barrier[2] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.state[kDirectSolved] = ok ? 1 : 0;
-    a.state[ok ? kDirectSolves : kDirectMisses] += 1;
-    a.state[kDirectApplied] += app;
+    a.stats[ok ? kStatDirectSolves : kStatDirectMisses] += 1;
+    a.stats[kStatDirectApplied] += app;
     // Given up once it has missed more often than not in this step: the
     // tries then cost no more than the solves before them have saved.
-    if (!ok && a.state[kDirectMisses] > a.state[kDirectSolves]) a.state[kDirectFailed] = 1;
+    if (!ok && a.stats[kStatDirectMisses] > a.stats[kStatDirectSolves])
+      a.state[kDirectFailed] = *a.failed = 1;
   }
   if (!ok) return;  // the CG launched after this solves from the unchanged start
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nv; i += gridDim.x * blockDim.x)

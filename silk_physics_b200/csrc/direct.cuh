@@ -25,14 +25,11 @@ constexpr int kDirectMaxLevels = 12;
 constexpr int kDirectThreads = 1024;
 constexpr int kDirectMaxApplications = 4;
 
-// Words of DirectArgs::state.  The last three count over a step.
+// Words of DirectArgs::state.
 enum DirectState {
-  kDirectFailed = 0,    // no usable factors, or given up
-  kDirectSolved = 1,    // the last solve met its tolerance
-  kDirectSolves = 2,    // solves that met it
-  kDirectMisses = 3,    // solves that did not (left to the CG)
-  kDirectApplied = 4,   // applications of the factors
-  kDirectWords = 5
+  kDirectFailed = 0,  // no usable factors, or given up
+  kDirectSolved = 1,  // the last solve met its tolerance
+  kDirectWords = 2
 };
 
 struct DirectArgs {
@@ -59,6 +56,8 @@ struct DirectArgs {
   double* partials = nullptr;
   unsigned* barrier = nullptr;  // [count, err, blocks that left]
   int* state = nullptr;  // kDirectWords words
+  int* stats = nullptr;   // CgArgs::stats
+  int* failed = nullptr;  // AdmmControl::direct_failed
   int* fail = nullptr;   // kFail* word of the solver
   const int* skip = nullptr;
   const float* rel_tol_dev = nullptr;

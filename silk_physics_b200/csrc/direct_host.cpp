@@ -249,14 +249,6 @@ void DirectSystem::upload(const DirectPlan& P, const std::vector<DirectNodeDev>&
   CUDA_CHECK(cudaMemsetAsync(state_, 0, kDirectWords * sizeof(int), st));
 }
 
-void DirectSystem::begin_step(cudaStream_t st) {
-  factorisations_ = 0;
-  given_up_ = false;
-  if (usable_)
-    CUDA_CHECK(cudaMemsetAsync(state_ + kDirectSolves, 0,
-                               (kDirectWords - kDirectSolves) * sizeof(int), st));
-}
-
 void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* skip,
                              cudaStream_t st) {
   DirectFactorArgs a;
@@ -296,7 +288,7 @@ void DirectSystem::factorize(const double* Lvals, const float* dyn, const int* s
   }
 }
 
-void DirectSystem::solve(const CgArgs& cg, cudaStream_t st) {
+void DirectSystem::solve(const CgArgs& cg, int* failed, cudaStream_t st) {
   DirectArgs a = args_;
   a.nslices = cg.nslices;
   a.sl_ptr = cg.sl_ptr;
@@ -307,6 +299,8 @@ void DirectSystem::solve(const CgArgs& cg, cudaStream_t st) {
   a.b = cg.b;
   a.x = cg.x;
   a.fail = cg.fail;
+  a.stats = cg.stats;
+  a.failed = failed;
   a.skip = cg.skip;
   a.rel_tol_dev = cg.rel_tol_dev;
   a.rel_tol = cg.rel_tol;

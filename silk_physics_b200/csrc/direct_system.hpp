@@ -17,15 +17,17 @@ class DirectSystem {
   void give_up() { given_up_ = true; }
   // Factorises L + diag(dyn) (kernels return at entry once *skip is set).
   void factorize(const double* Lvals, const float* dyn, const int* skip, cudaStream_t st);
-  // Solves into a.x, to the tolerance of the CG solve `cg` stands for.
-  void solve(const CgArgs& cg, cudaStream_t st);
+  // Solves into a.x, to the tolerance of the CG solve `cg` stands for; sets
+  // *failed where it has no factors or gives up.
+  void solve(const CgArgs& cg, int* failed, cudaStream_t st);
   // Set when the last solve met its tolerance (the CG then has nothing to do).
   const int* solved() const { return state_ + kDirectSolved; }
-  // Counts over a step: cleared on `st`, read from state() (kDirectWords
-  // words on the device).
-  void begin_step(cudaStream_t st);
-  const int* state() const { return state_; }
-  int factorisations() const { return factorisations_; }
+  const int* state() const { return state_; }  // kDirectWords words on the device
+  void begin_step() {
+    factorisations_ = 0;
+    given_up_ = false;
+  }
+  int factorisations() const { return factorisations_; }  // queued in this step
   // Compulsory DRAM bytes of one application: the factors once, the matrix
   // rows and the vectors of its residual.
   double application_bytes() const { return application_bytes_; }

@@ -126,8 +126,12 @@ struct CgArgs {
   long long* trace = nullptr;
 };
 
-// Per-cloth CG statistics words (CgArgs::stats).
-constexpr int kCgStats = 6;
+// Per-cloth statistics words of a step (CgArgs::stats); the last three are
+// the direct form's.
+constexpr int kStatDirectSolves = 6;   // systems it solved
+constexpr int kStatDirectMisses = 7;   // systems it left to the CG
+constexpr int kStatDirectApplied = 8;  // applications of its factors
+constexpr int kCgStats = 9;
 // Halo slots per block of the resident CG kernel (shared memory after the
 // block's own kResThreads slots).
 constexpr int kResHalo = 1024;

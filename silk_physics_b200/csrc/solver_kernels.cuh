@@ -75,7 +75,9 @@ struct AdmmControl {
   // Blocks of the running vertex step that have stored their partials; the
   // last one runs the convergence test and sets it back to 0.
   unsigned ticket;
-  int pad[5];
+  // A cloth's direct form had no factors or gave up (direct_solve_kernel).
+  int direct_failed;
+  int pad[4];
 };
 static_assert(sizeof(AdmmControl) == 64, "one control block of 64 bytes");
 

@@ -1082,7 +1082,7 @@ void World::cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStrea
     if (ev) CUDA_CHECK(cudaEventRecord(ev->first, st));
     auto* dv = opt.profile ? next_event_pair(events_direct, events_direct_used) : nullptr;
     if (dv) CUDA_CHECK(cudaEventRecord(dv->first, st));
-    c.dev.direct->solve(a, st);
+    c.dev.direct->solve(a, &ctl.p->direct_failed, st);
     if (dv) CUDA_CHECK(cudaEventRecord(dv->second, st));
     a.solved = c.dev.direct->solved();
     launch();
@@ -1400,7 +1400,7 @@ bool World::admm_solve() {
   if (ran > kDirectFrom) step_direct_ = true;
   // Where the matrix had no factors or the tolerance was out of reach, the
   // step's later ADMM solves do not factorise for it again.
-  if (factored) {
+  if (factored && ctl_host_.direct_failed) {
     std::vector<int> failed(cloths.size(), 0);
     for (size_t k = 0; k < cloths.size(); ++k)
       if (cloths[k]->dev.direct->usable())
@@ -1438,7 +1438,7 @@ silk_status World::solver_step() {
     int nv = nv_total;
     for (auto& c : cloths) {
       c->dev.stats.zero(st);
-      if (c->dev.direct) c->dev.direct->begin_step(st);
+      if (c->dev.direct) c->dev.direct->begin_step();
     }
     events_used = 0;
     events_factor_used = 0;
@@ -1560,13 +1560,6 @@ silk_status World::solver_step() {
     for (size_t k = 0; k < cloths.size(); ++k)
       CUDA_CHECK(cudaMemcpyAsync(&cgs[kCgStats * k], cloths[k]->dev.stats.p,
                                  kCgStats * sizeof(int), cudaMemcpyDeviceToHost, st));
-    std::vector<int> direct(kDirectWords * cloths.size(), 0);
-    for (size_t k = 0; k < cloths.size(); ++k) {
-      const DirectSystem* d = cloths[k]->dev.direct.get();
-      if (d && d->factorisations() > 0)
-        CUDA_CHECK(cudaMemcpyAsync(&direct[kDirectWords * k], d->state(),
-                                   kDirectWords * sizeof(int), cudaMemcpyDeviceToHost, st));
-    }
     sync();
     for (size_t k = 0; k < cloths.size(); ++k) {
       const int* q = &cgs[kCgStats * k];
@@ -1580,12 +1573,11 @@ silk_status World::solver_step() {
       stats.extrapolated_starts += q[4];
       stats.learned_iterate_starts += q[5];
       if (const DirectSystem* d = cloths[k]->dev.direct.get()) {
-        const int* s = &direct[kDirectWords * k];
         direct_stats.factorisations += d->factorisations();
-        direct_stats.solves += s[kDirectSolves];
-        direct_stats.misses += s[kDirectMisses];
-        direct_stats.applications += s[kDirectApplied];
-        direct_stats.application_bytes += s[kDirectApplied] * d->application_bytes();
+        direct_stats.solves += q[kStatDirectSolves];
+        direct_stats.misses += q[kStatDirectMisses];
+        direct_stats.applications += q[kStatDirectApplied];
+        direct_stats.application_bytes += q[kStatDirectApplied] * d->application_bytes();
       }
       if (opt.profile) {
         double bpi = opt.mas_bf16 ? cloths[k]->dev.bytes_per_iter_bf16
