@@ -84,16 +84,6 @@ __global__ void __launch_bounds__(256) direct_add_kernel(DirectFactorArgs a,
   }
 }
 
-// 1 / p for the pivots: the hardware's approximation (about 20 bits) and two
-// Newton steps, each squaring the relative error.  A pivot that is zero,
-// negative or not finite gives no positive finite result and is refused.
-__device__ __forceinline__ double reciprocal(double p) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
-  r = fma(r, fma(-p, r, 1.0), r);
-  return fma(r, fma(-p, r, 1.0), r);
-}
-
 // Symmetric Gauss-Jordan of a 32 x 32 block by one warp: lane j holds column j
 // in registers.  A pivot publishes its row (by symmetry its column) through
 // shared memory, one double per lane.  The next pivot's row is updated first,
@@ -102,7 +92,7 @@ __device__ __forceinline__ double reciprocal(double p) {
 __device__ bool invert_warp(double (&x)[kP], double (*row)[kP], int lane) {
   bool good = true;
   row[0][lane] = x[0];
-  double p = __shfl_sync(0xffffffffu, x[0], 0), inv = reciprocal(p);
+  double p = __shfl_sync(0xffffffffu, x[0], 0), inv = __drcp_rn(p);
   __syncwarp();
 #pragma unroll
   for (int k = 0; k < kP; ++k) {
@@ -117,7 +107,7 @@ __device__ bool invert_warp(double (&x)[kP], double (*row)[kP], int lane) {
       x[k + 1] = fma(-s[k + 1], f, own ? 0.0 : x[k + 1]);
       row[(k + 1) & 1][lane] = x[k + 1];
       p = __shfl_sync(0xffffffffu, x[k + 1], k + 1);
-      next = reciprocal(p);
+      next = __drcp_rn(p);
     }
 #pragma unroll
     for (int i = 0; i < kP; ++i)
