@@ -2431,9 +2431,9 @@ int CollisionSystem::append_active(float time, float dact) {
   I.colors.alloc(total);
   I.colors.zero(st);
   I.col_info.zero(st);
+  const int dev = current_device();
   {
     static PerDevice<int> coop;
-    const int dev = current_device();
     const int max_coop = coop.get(dev, [dev] {
       int sms = 0, per = 0;
       CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2533,6 +2533,13 @@ int CollisionSystem::append_active(float time, float dact) {
     gs_rec_kernel<<<div_up(total, 256), 256, 0, st>>>(I.gs_cc.p, I.gs_place.p, total,
                                                       I.col_info.p, I.gs_rec.p);
     SILK_LAUNCHED();
+    static PerDevice<bool> opted;
+    opted.get(dev, [] {
+      for (auto* k : {contact_gs_flow_kernel<true>, contact_gs_flow_kernel<false>})
+        CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kGsBlockSmemMax));
+      return true;
+    });
     I.gs_ready = true;
   }
   // The one host read of the contact build's colouring and layout.
@@ -2563,13 +2570,6 @@ void CollisionSystem::contact_solve_launch() {
   const size_t both = pos + (size_t)I.n_contacts * sizeof(float4);
   if (I.gs_ready && w_.opt.contact_gs_form != 1 && pos <= kGsBlockSmemMax &&
       I.n_contacts <= kGsContactsPerColour * I.n_colors) {
-    static PerDevice<bool> opted;
-    opted.get(current_device(), [] {
-      for (auto* k : {contact_gs_flow_kernel<true>, contact_gs_flow_kernel<false>})
-        CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kGsBlockSmemMax));
-      return true;
-    });
     const bool shared = both <= kGsBlockSmemMax;
     // About six batches a warp: fewer leave warps polling beside the ones
     // that work, more put contacts that could run behind ones that wait
