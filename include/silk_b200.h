@@ -107,7 +107,8 @@ typedef struct {
                                  iterate model is loaded, its prediction of
                                  the next ADMM iterate as the start of every
                                  later CG solve (from the third of an ADMM
-                                 solve on) */
+                                 solve on); not computed for systems that the
+                                 direct form takes */
   int32_t capture_samples;    /* bit 1: record first-solve training samples;
                                  bit 2: record iterate-model training samples
                                  (256 vertices per ADMM iteration) */

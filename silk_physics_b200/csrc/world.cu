@@ -1038,7 +1038,7 @@ float World::warm_sigma() const {
 void World::cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStream_t st) {
   CgArgs a = c.dev.cg;
   a.first_solve = first ? 1 : 0;
-  if (first && has_model && opt.learned_warm_start) {
+  if (first && warm_ready_) {
     a.x_alt = xpred.p + c.voff;
     a.alt_stat = 3;
   } else if (!first && iter_ready) {
@@ -1216,6 +1216,12 @@ silk_status World::get_cloth_velocity(uint32_t h, float* out, int64_t n) {
   return SILK_OK;
 }
 
+bool World::all_direct() const {
+  for (const auto& c : cloths)
+    if (!c->dev.direct || !c->dev.direct->usable()) return false;
+  return true;
+}
+
 bool World::admm_solve() {
   NvtxRange admm_range("ADMM solve");
   SolverView s = view();
@@ -1291,7 +1297,12 @@ bool World::admm_solve() {
       sync();
       if (ctl_host_.done) break;
     }
-    if (it != 0 && (iter_model || iter_capture)) {
+    // Starts are offered to the CG alone: not computed where every system
+    // goes to factors that are at hand (a miss then starts from x; 10 ms of a
+    // 104 ms step of the learned 80 x 80 scene, read by nothing).
+    const bool starts = !(direct && all_direct());
+    iter_ready = admm_ext_ready = false;
+    if (it != 0 && ((iter_model && starts) || iter_capture)) {
       // x holds x_(it-1); slots (it-1) % 3 and (it-2) % 3 hold x_(it-2) and
       // x_(it-3) from the previous iterations.
       if (it >= 3) {
@@ -1308,7 +1319,7 @@ bool World::admm_solve() {
       // Extrapolated start: from the third solve on, 2 x_k - x_(k-1) of the
       // last two iterates of this ADMM solve (the first solve starts from the
       // outer state, whose step to x_1 is not an ADMM iterate difference).
-      if (opt.admm_extrapolated_start && it >= 2) {
+      if (opt.admm_extrapolated_start && starts && it >= 2) {
         if (admm_prev.n < (size_t)nv_total) {
           admm_prev.alloc(nv_total);
           admm_ext.alloc(nv_total);
@@ -1492,12 +1503,14 @@ silk_status World::solver_step() {
       launch_predict(nv, g.dt, make_float4(g.acceleration_x, g.acceleration_y, g.acceleration_z, 0.f),
                      outer.p, outer_v.p, x.p, st);
       warm_first_ = oit == 0;
-      if (warm_active()) {
+      warm_ready_ = has_model && opt.learned_warm_start &&
+                    !(opt.cg_form == 0 && step_direct_ && all_direct());
+      if (warm_ready_ || (opt.capture_samples & 1)) {
         const float sigma = warm_sigma();
         CUDA_CHECK(cudaMemcpyAsync(ypred.p, x.p, nv * sizeof(float4), cudaMemcpyDeviceToDevice, st));
         warm_features(nv, outer.p, hist1.p, hist2.p, ypred.p, pin_flag.p, ring_off.p, ring.p,
                       1.0f / sigma, warm_feat.p, st);
-        if (has_model && opt.learned_warm_start) {
+        if (warm_ready_) {
           MlpDev m{mlp_params.p, mlp_image_buf.p, cg_fail.p};
           warm_predict(m, nv, warm_feat.p, ypred.p, sigma, mlp_out.p, xpred.p, st);
         }

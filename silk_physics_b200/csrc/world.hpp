@@ -262,6 +262,7 @@ class World {
   bool iter_ready = false;  // iter_pred holds a prediction for the coming solve
   bool has_model = false;
   bool samples_valid = false;
+  bool warm_ready_ = false;  // xpred holds a prediction for the coming first solve
   bool warm_first_ = false;  // the current outer iteration is the step's first
   int pinned_dof = 0;
   silk_profile prof{};
@@ -289,15 +290,13 @@ class World {
   void build_cloth_device(Cloth& c);
   void build_resident_layout(Cloth& c);
   void upload_pins();
+  bool all_direct() const;  // every cloth has a usable direct system
   void factorize(Cloth& c, cudaStream_t st);
   void cg_solve(Cloth& c, float rel_tol, bool first, bool direct, cudaStream_t st);
   void ensure_cloth_streams(size_t n);
   std::vector<cudaStream_t> cloth_streams_;  // per-cloth CG streams (multi-cloth worlds)
   std::vector<cudaEvent_t> cloth_done_;
   cudaEvent_t fork_ev_ = nullptr;
-  bool warm_active() const {
-    return (has_model && opt.learned_warm_start) || (opt.capture_samples & 1);
-  }
   float warm_sigma() const;
   bool admm_solve();  // false on divergence
   void sync();

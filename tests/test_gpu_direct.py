@@ -1,5 +1,7 @@
 """The direct form of long ADMM solves (nested-dissection factors applied with
 refinement) against the CG it replaces."""
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -281,3 +283,37 @@ def test_two_cloths_in_contact_match_cg(sizes):
         own = max(np.abs(o[0][k] - out[3][0][k]).max() for o in out[1:3])
         print(f"{sizes[k]}: {out[0][1].contacts} contacts, direct {err:.2e}, CG {own:.2e}")
         assert err <= max(3.0 * own, 5e-6)
+
+
+@pytest.mark.parametrize("learned, extrapolated", [(True, False), (False, True), (True, True)])
+def test_no_starts_for_systems_solved_directly(learned, extrapolated):
+    """The learned and extrapolated starts are offered to the CG alone: an
+    iteration whose systems are solved directly launches what the plain one
+    does, and the steps before the threshold start as before."""
+    V, F = S.grid_sheet(24, jitter=1e-4, seed=3)
+
+    def run(inner, **opts):
+        w = N.World()
+        assert w.init()
+        assert w.set_global_config(N.GlobalConfig(max_inner_iteration=inner, admm_abs_tol=0.0,
+                                                  admm_rel_tol=0.0))
+        assert w.set_solver_options(N.SolverOptions(fixed_linear_rel_tol=1e-6, **opts))
+        r, h = w.add_cloth(N.ClothConfig(), N.CollisionConfig(
+            is_collision_on=False, is_self_collision_on=False), V, F, S.top_corner_pins(24))
+        assert r
+        if opts.get("learned_warm_start"):
+            assert w.set_warm_start_model(learned_model)
+        for _ in range(2):  # the second step has the direct system from the start
+            r = w.solver_step()
+            assert r, r.to_string()
+        st = w.step_stats()
+        assert st.cg_solves == DIRECT_FROM - 1
+        return st.kernel_launches, st.learned_iterate_starts + st.extrapolated_starts
+
+    from silk_physics_b200 import learned as L
+    learned_model = L.load(str(Path(N.__file__).resolve().parent / "models" / "warm_start.npy"))
+    opts = dict(learned_warm_start=learned, admm_extrapolated_start=extrapolated)
+    plain = [run(k)[0] for k in (24, 40)]
+    other = [run(k, **opts) for k in (24, 40)]
+    assert other[1][0] - other[0][0] == plain[1] - plain[0]
+    assert other[0][0] > plain[0] and other[0][1] > 0
