@@ -83,7 +83,8 @@ typedef struct {
   float fixed_linear_rel_tol; /* > 0: CG relative tolerance fixed (1e-5 in
                                  the headline benchmark); 0: adaptive rule of
                                  admm_solver.cu:228-233 */
-  int32_t cg_max_iter;        /* 1000 (mas_cg_solver.cuh:25) */
+  int32_t cg_max_iter;        /* 1000 (mas_cg_solver.cuh:25); bounds the CG, not
+                                 the direct form (see cg_form) */
   int32_t mas_bf16;           /* 0: FP32 bank inverses; 1: BF16 storage */
   int32_t profile;            /* 1: time the CG kernel with CUDA events;
                                  2: also record the CG phase trace */

@@ -10,7 +10,7 @@ namespace silkb {
 
 // Bits of the solver failure word (World::cg_fail), read by the ADMM
 // convergence test and reported as IterativeSolveFail.
-constexpr int kFailBarrier = 1;   // a grid-barrier wait of a CG kernel gave up
+constexpr int kFailBarrier = 1;   // a grid-barrier wait of the CG or a direct solve gave up
 constexpr int kFailMasPivot = 2;  // a MAS bank had a zero or non-finite pivot
 constexpr int kFailContactWait = 4;  // a contact Gauss-Seidel wait gave up
 

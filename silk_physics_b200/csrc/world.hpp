@@ -19,10 +19,14 @@ namespace silkb {
 class DirectSystem;
 
 // ADMM iteration from which a solve's systems go to the direct form, and with
-// them those of every later ADMM solve of the step.  A factorisation costs
-// about four CG solves (0.9 ms against 0.24 at 6,400 vertices, 6.5 against
-// 1.7 at 100K), so short solves stay with the CG; one that has come this far
-// is likely to take as many iterations again.
+// them those of every later ADMM solve of the step.  A factorisation costs one
+// to three CG solves (ms: 0.14 and 0.14 at 144 vertices, 0.49 and 0.21 at
+// 1,600, 0.85 and 0.44 at 6,400, 4.1 and 1.9 at 100K) and a direct solve a
+// fifth of one or less, so the break-even lies a few iterations in; the plan,
+// built in a cloth's first such step, costs more (4 ms of host time at 6,400
+// vertices, 100 at 100K).  16 lies above the ten iterations of the small
+// configuration, whose CG counts the tests hold to; lower lines were not
+// measured.
 constexpr int kDirectFrom = 16;
 
 // Owning device allocation.
