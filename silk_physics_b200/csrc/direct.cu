@@ -581,11 +581,13 @@ __global__ void __launch_bounds__(kDirectThreads, 1) direct_solve_kernel(DirectA
     a.barrier[0] = a.barrier[2] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.state[kDirectSolved] = ok ? 1 : 0;
-    a.stats[ok ? kStatDirectSolves : kStatDirectMisses] += 1;
-    a.stats[kStatDirectApplied] += app;
+    // Reductions whose result is not waited for, but for a miss.
+    atomicAdd(a.stats + kStatDirectApplied, app);
+    if (ok)
+      atomicAdd(a.stats + kStatDirectSolves, 1);
     // Given up once it has missed more often than not in this step: the
     // tries then cost no more than the solves before them have saved.
-    if (!ok && a.stats[kStatDirectMisses] > a.stats[kStatDirectSolves])
+    else if (atomicAdd(a.stats + kStatDirectMisses, 1) >= a.stats[kStatDirectSolves])
       a.state[kDirectFailed] = *a.failed = 1;
   }
   if (!ok) return;  // the CG launched after this solves from the unchanged start
